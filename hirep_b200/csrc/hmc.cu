@@ -15,6 +15,7 @@
 
 #include "dirac.cuh"
 #include "rng.cuh"
+#include "suN.cuh"
 
 namespace hrgpu {
 
@@ -68,7 +69,7 @@ __device__ __forceinline__ double fund_project(const CMat<N> &w, const double2 *
   return s * 2.0;
 }
 
-// force0: mom(x,mu) += coeff * proj(U(x,mu) S(x,mu)^+), S the six staples
+// force0: mom(x,mu) += coeff * proj(U(x,mu) S(x,mu)^+), S the six staples (NG > 4)
 template <int N>
 __global__ void k_force0(double *mom, const double2 *Ug, const double2 *gT, Geo g, int dimg, double coeff) {
   const long d = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -107,7 +108,223 @@ __global__ void k_force0(double *mom, const double2 *Ug, const double2 *gT, Geo 
   for (int A = 0; A < dimg; A++) mom[((long)mu * dimg + A) * lp + d] += coeff * fund_project<N>(b, gT, A);
 }
 
-// U(x,mu) <- exp(dt sum_A mom_A iT_A) U(x,mu)   (ExpX)
+// force0 for NG <= 4: the staple sum, one staple's product and a row or column of
+// the streamed links are all that is held (two N x N matrices in registers), each
+// link element loaded once per product.  A block is 32 sites x the 4 directions,
+// one warp each, so the links that the directions share (44 of the 76 a site reads
+// are different) and the x neighbours hit L1.
+// What bounds it: the link loads from L1/L2 (76 links of 16 N^2 bytes a site).
+template <int N>
+__global__ void __launch_bounds__(128) k_force0_r(double *mom, const double2 *Ug, Geo g, double coeff) {
+  const long d = (long)blockIdx.x * 32 + (threadIdx.x & 31);
+  const int mu = threadIdx.x >> 5;
+  if (!real_site(g, d)) return;
+  const long lp = 2L * g.ld;
+  int t, x, y, z;
+  dev_coords(g, (int)d, t, x, y, z);
+  const long xpmu = site_at(g, t, x, y, z, mu, 1, mu, 0);
+  double2 S[N][N], T[N][N];
+  mzero<N>(S);
+#pragma unroll 1
+  for (int i = 1; i < 4; i++) {
+    const int nu = (mu + i) & 3;
+    const long xpnu = site_at(g, t, x, y, z, nu, 1, nu, 0), xmnu = site_at(g, t, x, y, z, nu, -1, nu, 0);
+    const long xpmumnu = site_at(g, t, x, y, z, mu, 1, nu, -1);
+    // up: U(x,nu) U(x+nu,mu) U(x+mu,nu)^+
+    mul_ll<N, false, false>(T, link_at<N>(Ug, nu, d, lp), link_at<N>(Ug, mu, xpnu, lp));
+    mac_rl<N, true>(S, T, link_at<N>(Ug, nu, xpmu, lp));
+    // down: U(x-nu,nu)^+ U(x-nu,mu) U(x+mu-nu,nu)
+    mul_ll<N, true, false>(T, link_at<N>(Ug, nu, xmnu, lp), link_at<N>(Ug, mu, xmnu, lp));
+    mac_rl<N, false>(S, T, link_at<N>(Ug, nu, xpmumnu, lp));
+  }
+  // U S^+
+  const LinkPtr<N> u = link_at<N>(Ug, mu, d, lp);
+  mzero<N>(T);
+#pragma unroll
+  for (int k = 0; k < N; k++)
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const double2 uk = u(i, k);
+#pragma unroll
+      for (int j = 0; j < N; j++) cmac(T[i][j], uk, cconj(S[j][k]));
+    }
+  double *m = mom + (long)mu * (N * N - 1) * lp + d;
+  algebra_project<N>(T, [&](int A, double f) { m[(long)A * lp] += coeff * f; });
+}
+
+// update_gauge_field for NG <= 4.  X = dt sum_A mom_A iT_A = i H with H Hermitian
+// and traceless, so by the Cayley-Hamilton theorem H^N is a combination of lower
+// powers whose coefficients are traces of H^2, H^3 and H^4, and the exponential is
+// sum_k f_k H^k with k < N: the Taylor series runs over the N coefficients of
+// H^n / n! (a scalar recursion, to n = 19) instead of over N x N products.  H is
+// scaled by 2^-s to |H|_F <= 1 first and the result squared s times (s = 0 for any
+// step size in use), so the series' truncation (1/20! = 4e-19) and its rounding
+// stay below FP64's.  H, H^2 and H^3 are Hermitian: N^2 reals each.
+// One thread per link.  With k_force0_r, against local-memory Taylor products and
+// staple matrices (0.99 + 1.41 ms), the step of fermion force, gauge force, link
+// update and one operator at 16^4 SU(4) antisymmetric goes from 2.90 to 0.67 ms.
+template <int N>
+__global__ void __launch_bounds__(128) k_update_gauge_r(double2 *Ug, const double *mom, Geo g, double dt) {
+  const long d = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int mu = blockIdx.y;
+  if (d >= 2L * g.ld || !real_site(g, d)) return;
+  const long lp = 2L * g.ld;
+  const double *m = mom + (long)mu * (N * N - 1) * lp + d;
+  // the lower triangle of H, real diagonal
+  double hd[N], h2d[N];
+  double2 ho[N][N], h2o[N][N];  // [i][j], j < i
+#pragma unroll
+  for (int i = 0; i < N; i++) hd[i] = 0.0;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j < i) {
+        // T_(i,j) symmetric, T_(j,i) antisymmetric: element (j, i) is (h_s + i h_a) / 2
+        const double hs = m[(long)gen_index<N>(i, j) * lp], ha = m[(long)gen_index<N>(j, i) * lp];
+        ho[i][j] = make_double2(0.5 * dt * hs, -0.5 * dt * ha);
+      }
+    if (i > 0) {
+      const double q = 0.5 * sqrt(2.0 / ((double)i * (i + 1.0))) * dt * m[(long)gen_index<N>(i, i) * lp];
+#pragma unroll
+      for (int k = 0; k < N; k++)
+        if (k < i) hd[k] += q;
+      hd[i] -= (double)i * q;
+    }
+  }
+  double t2 = 0.0;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    t2 += hd[i] * hd[i];
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j < i) t2 += 2.0 * (ho[i][j].x * ho[i][j].x + ho[i][j].y * ho[i][j].y);
+  }
+  int sq = 0;
+  while (t2 > 1.0 && sq < 60) {
+    t2 *= 0.25;
+    sq++;
+  }
+  const double sc = ldexp(1.0, -sq);
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    hd[i] *= sc;
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j < i) ho[i][j] = make_double2(sc * ho[i][j].x, sc * ho[i][j].y);
+  }
+  auto H = [&](int i, int j) { return i == j ? make_double2(hd[i], 0.0) : (j < i ? ho[i][j] : cconj(ho[j][i])); };
+  double t3 = 0.0, t4 = 0.0;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j <= i) {
+        double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < N; k++) cmac(s, H(i, k), H(k, j));
+        if (i == j) {
+          h2d[i] = s.x;
+          t3 += s.x * hd[i];
+          t4 += s.x * s.x;
+        } else {
+          h2o[i][j] = s;
+          t3 += 2.0 * (s.x * ho[i][j].x + s.y * ho[i][j].y);
+          t4 += 2.0 * (s.x * s.x + s.y * s.y);
+        }
+      }
+  auto H2 = [&](int i, int j) { return i == j ? make_double2(h2d[i], 0.0) : (j < i ? h2o[i][j] : cconj(h2o[j][i])); };
+  // H^N = sum_k c_k H^k (Newton's identities with Tr H = 0)
+  double c[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) c[k] = 0.0;
+  if (N == 2) c[0] = 0.5 * t2;
+  if (N == 3) {
+    c[0] = t3 * (1.0 / 3.0);
+    c[N > 2 ? 1 : 0] = 0.5 * t2;
+  }
+  if (N == 4) {
+    c[0] = 0.25 * t4 - 0.125 * t2 * t2;
+    c[N > 2 ? 1 : 0] = t3 * (1.0 / 3.0);
+    c[N > 2 ? 2 : 0] = 0.5 * t2;
+  }
+  // f_k = sum_n i^n u_k(n), H^n / n! = sum_k u_k(n) H^k
+  double2 f[N];
+  double u[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    f[k] = make_double2(k == 0 ? 1.0 : 0.0, 0.0);
+    u[k] = k == 0 ? 1.0 : 0.0;
+  }
+#pragma unroll
+  for (int n = 1; n < 20; n++) {
+    const double inv = 1.0 / n, top = u[N - 1];
+#pragma unroll
+    for (int k = N - 1; k > 0; k--) u[k] = inv * fma(c[k], top, u[k - 1]);
+    u[0] = inv * c[0] * top;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+      if ((n & 3) == 0) f[k].x += u[k];
+      if ((n & 3) == 1) f[k].y += u[k];
+      if ((n & 3) == 2) f[k].x -= u[k];
+      if ((n & 3) == 3) f[k].y -= u[k];
+    }
+  }
+  double2 E[N][N];
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j <= i) {
+        double2 h3 = make_double2(0.0, 0.0);
+        if (N == 4) {
+#pragma unroll
+          for (int k = 0; k < N; k++) cmac(h3, H(i, k), H2(k, j));
+        }
+        double2 a = make_double2(0.0, 0.0), b = a;  // elements (i, j) and (j, i)
+        auto add = [&](double2 fk, double2 hk) {
+          cmac(a, fk, hk);
+          cmac(b, fk, cconj(hk));
+        };
+        if (i == j) a = b = f[0];
+        add(f[1], H(i, j));
+        if (N > 2) add(f[N > 2 ? 2 : 1], H2(i, j));
+        if (N > 3) add(f[N > 3 ? 3 : 1], h3);
+        E[i][j] = a;
+        E[j][i] = i == j ? a : b;
+      }
+  for (; sq > 0; sq--) {
+    double2 Q[N][N];
+    mzero<N>(Q);
+#pragma unroll
+    for (int k = 0; k < N; k++)
+#pragma unroll
+      for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = 0; j < N; j++) cmac(Q[i][j], E[i][k], E[k][j]);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+      for (int j = 0; j < N; j++) E[i][j] = Q[i][j];
+  }
+  // E U, a column of U at a time: the column's elements are read before they are written
+  double2 *U = Ug + (long)mu * N * N * lp + d;
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    double2 v[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] = U[(long)(k * N + j) * lp];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int k = 0; k < N; k++) cmac(s, E[i][k], v[k]);
+      U[(long)(i * N + j) * lp] = s;
+    }
+  }
+}
+
+// U(x,mu) <- exp(dt sum_A mom_A iT_A) U(x,mu)   (ExpX), NG > 4
 template <int N>
 __global__ void k_update_gauge(double2 *Ug, const double *mom, const double2 *gT, Geo g, int dimg, double dt) {
   const long d = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -279,6 +496,26 @@ __global__ void k_add(double *a, const double *b, long n) {
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) a[i] += b[i];
 }
 
+// NG <= SUN_MAX: the register kernels
+#define HR_SUN_DISPATCH(NGV, CALL)                      \
+  do {                                                  \
+    if ((NGV) == 2) { constexpr int N_ = 2; CALL; }      \
+    else if ((NGV) == 3) { constexpr int N_ = 3; CALL; } \
+    else { constexpr int N_ = 4; CALL; }                 \
+  } while (0)
+
+// NG > SUN_MAX: the kernels with local-memory matrices
+#define HR_LARGE_NG_DISPATCH(NGV, CALL)                                                 \
+  do {                                                                                  \
+    switch (NGV) {                                                                      \
+      case 5: { constexpr int N_ = 5; CALL; } break;                                     \
+      case 6: { constexpr int N_ = 6; CALL; } break;                                     \
+      case 7: { constexpr int N_ = 7; CALL; } break;                                     \
+      case 8: { constexpr int N_ = 8; CALL; } break;                                     \
+      default: set_error("no HMC kernel for NG=%d", (int)(NGV)); return HRGPU_E_NF;       \
+    }                                                                                   \
+  } while (0)
+
 #define HR_NG_DISPATCH(NGV, CALL)                                                       \
   do {                                                                                  \
     switch (NGV) {                                                                      \
@@ -411,7 +648,10 @@ int hrgpu_force0(double dt, double beta) {
   HR_REQUIRE(L.have_fund, HRGPU_E_STATE, "force0: no fundamental gauge field");
   const Geo g = make_geo();
   const double coeff = -dt * beta / L.ng;
-  HR_NG_DISPATCH(L.ng, (k_force0<N_><<<dim3(nb128(2L * L.ld), 4), 128, 0, L.stream>>>(L.mom, L.Ug, g_gT, g, L.dimg, coeff)));
+  if (L.ng <= SUN_MAX)
+    HR_SUN_DISPATCH(L.ng, (k_force0_r<N_><<<(unsigned)(2L * L.ld / 32), 128, 0, L.stream>>>(L.mom, L.Ug, g, coeff)));
+  else
+    HR_LARGE_NG_DISPATCH(L.ng, (k_force0<N_><<<dim3(nb128(2L * L.ld), 4), 128, 0, L.stream>>>(L.mom, L.Ug, g_gT, g, L.dimg, coeff)));
   HR_LAUNCH_CHECK();
   return 0;
 }
@@ -429,7 +669,10 @@ int hrgpu_update_gauge_field(double dt) {
   if (int rc = hmc_setup()) return rc;
   HR_REQUIRE(L.have_fund, HRGPU_E_STATE, "update_gauge_field: no fundamental gauge field");
   const Geo g = make_geo();
-  HR_NG_DISPATCH(L.ng, (k_update_gauge<N_><<<dim3(nb128(2L * L.ld), 4), 128, 0, L.stream>>>(L.Ug, L.mom, g_gT, g, L.dimg, dt)));
+  if (L.ng <= SUN_MAX)
+    HR_SUN_DISPATCH(L.ng, (k_update_gauge_r<N_><<<dim3(nb128(2L * L.ld), 4), 128, 0, L.stream>>>(L.Ug, L.mom, g, dt)));
+  else
+    HR_LARGE_NG_DISPATCH(L.ng, (k_update_gauge<N_><<<dim3(nb128(2L * L.ld), 4), 128, 0, L.stream>>>(L.Ug, L.mom, g_gT, g, L.dimg, dt)));
   HR_LAUNCH_CHECK();
   fund_links_changed();
   // reunitarise every 17th call, as the reference's counter does (field_update.c:45-57)
