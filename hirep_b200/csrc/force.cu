@@ -612,9 +612,14 @@ static int launch_force_expclover(double2 *clf, const double2 *cl, const double2
   return 0;
 }
 
-// force_clover_core (force_fermion_core.c:282-379): one thread per (site, mu)
+// force_clover_core (force_fermion_core.c:282-379): one thread per (site, mu), the
+// products in the fermion representation: for the groups that cforce.cu does not
+// cover, represented links uploaded by themselves, and links that are not unitary.
+// run: when non-null, nothing is done unless *run is set (cforce.cu's check failed)
 template <int N, bool REAL>
-__global__ void k_force_clover_core(double *fsum, const void *U, const double2 *clf, Geo g, ProjTab P, double coeff) {
+__global__ void k_force_clover_core(double *fsum, const void *U, const double2 *clf, Geo g, ProjTab P, double coeff,
+                                    const int *run) {
+  if (run && !*run) return;
   long d = (long)blockIdx.x * blockDim.x + threadIdx.x;
   int mu = blockIdx.y;
   if (d >= 2L * g.ld) return;
@@ -857,7 +862,9 @@ int fermion_force_finish(double dt) {
   const double coeff = dt * (L.repr_norm2 / L.fund_norm2) * (1. / 8.) * L.csw;
   Geo g = make_geo();
   const long n = 2L * L.ld;
-  HR_NF_DISPATCH(L.real, L.nf, (k_force_clover_core<N_, R_><<<dim3(nb(n, 64), 4), 64, 0, L.stream>>>(L.force_sum, L.U, L.cl_force, g, proj(), coeff)));
+  int *run = nullptr;
+  if (const int rc = clover_force_fund(coeff, &run); rc > 0) return rc;
+  HR_NF_DISPATCH(L.real, L.nf, (k_force_clover_core<N_, R_><<<dim3(nb(n, 64), 4), 64, 0, L.stream>>>(L.force_sum, L.U, L.cl_force, g, proj(), coeff, run)));
   HR_LAUNCH_CHECK();
   return 0;
 }

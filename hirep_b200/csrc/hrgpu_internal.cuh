@@ -67,6 +67,7 @@ struct Lattice {
   float2 *Ugf = nullptr;  // fundamental links, float (for the FP32 hop of link modes 3 and 4)
   double2 *Ug = nullptr;  // fundamental links [4][ng*ng][2*ld]
   bool have_gauge = false, have_gauge_flt = false, have_fund = false;
+  bool fund_current = false;  // the represented links were made from the fundamental ones held
   // clover
   bool clover = false;
   bool expclover = false;         // WITH_EXPCLOVER: diagonal (4+m) exp(A/(4+m))
@@ -93,6 +94,7 @@ struct Lattice {
   int recon12 = 0;
   bool recon_allow = true;        // hrgpu_set_link_recon
   double2 *cl_force = nullptr;    // [6][nf*nf][2*ld]
+  double *cl_plaq = nullptr;      // clover force per plaquette link [6][4][dimg][2*ld], then a check word (cforce.cu)
   // algebra projection tables (sparse): for each generator A, entries (k=i*nf+j, coeff)
   int *d_proj_off = nullptr;      // [dimg+1]
   int *d_proj_k = nullptr;

@@ -64,7 +64,7 @@ static void free_ptr(void *p) {
 static void free_all() {
   cg_release();
   void *ptrs[] = {L.d_h2d, L.d_d2h, L.U, L.Uf, L.Ubf, L.Ug, L.Ugf, L.mom, L.cl_term, L.cl_dg, L.cl_od, L.cl_idg, L.cl_iod,
-                  L.cl_dg_f, L.cl_idg_f, L.cl_od_f, L.cl_iod_f, L.cl_ldet, L.force_sum, L.cl_force, L.d_proj_off,
+                  L.cl_dg_f, L.cl_idg_f, L.cl_od_f, L.cl_iod_f, L.cl_ldet, L.force_sum, L.cl_force, L.cl_plaq, L.d_proj_off,
                   L.d_proj_k, L.d_proj_c, L.d_projk_off, L.d_projk_A, L.d_projk_c, L.partials, L.d_scalars, L.tmp_o, L.tmp_e, L.tmp_e2, L.tmp_full,
                   L.tmp_full2, L.tmp_o_f, L.tmp_e_f, L.tmp_full_f, L.stage, L.hop_err, L.hopb_err};
   for (void *p : ptrs) free_ptr(p);
@@ -581,6 +581,7 @@ int hrgpu_gauge_set_f(const void *uf_host) {
   HR_CUDA(cudaMemcpyAsync(L.stage, uf_host, bytes, cudaMemcpyHostToDevice, L.stream));
   if (int rc = launch_links_in(L.U, L.stage, nel, L.real, 4)) return rc;
   L.have_gauge = true;
+  L.fund_current = false;
   if (int rc = detect_recon12()) return rc;
   if (int rc = hrgpu_assign_ud2u_f()) return rc;
   if (L.clover) {

@@ -209,6 +209,7 @@ int detect_recon12() {
 }
 
 void fund_links_changed() {
+  L.fund_current = false;
   if (L.recon12 >= 3) L.recon12 = 0;
 }
 
@@ -240,6 +241,7 @@ int hrgpu_represent_gauge_field(int bc_t_antiperiodic) {
   k_represent<<<dim3((unsigned)((n + 127) / 128), 4), 128, 0, L.stream>>>(L.U, L.Ug, L.ng, L.repr, g, bc_t_antiperiodic);
   HR_LAUNCH_CHECK();
   L.have_gauge = true;
+  L.fund_current = true;
   L.bc_t = bc_t_antiperiodic;
   if (int rc = set_recon12(bc_t_antiperiodic, true)) return rc;
   if (int rc = hrgpu_assign_ud2u_f()) return rc;

@@ -45,3 +45,53 @@ def test_update_gauge_field(ng, scale):
     ref = o.update_gauge_field(dt, u, mom)
     # one rounding of a unitary matrix per product, doubled by each squaring (up to 2^6 at scale 40)
     assert np.abs(lat.gauge_get() - ref).max() < 1e-14 * max(4.0, 4 * scale)
+
+
+GROUPS = [(2, O.FUND), (3, O.FUND), (4, O.FUND), (2, O.ADJ), (2, O.SYM), (3, O.SYM), (3, O.ASYM), (4, O.ASYM)]
+
+
+def clover_force_pair(o, lat, exp):
+    """The clover force (with the log-det force of the standard term) of the library and of the oracle."""
+    m, dt = 0.2, 0.7
+    x, y = (F.gaussian_spinor(3 + k, lat.V, lat.nf) for k in range(2))
+    for q in (o, lat):
+        (q.expclover_init if exp else q.clover_init)(1.3)
+        (o.set_mass if q is o else lat.set_dirac_mass)(m)
+        if q is o:
+            o.compute_clover_term()
+        q.fermion_force_begin()
+        if q is lat:
+            lat.force_fermion_core(lat.field(G.FULL, host=x), lat.field(G.FULL, host=y), 1, dt, 1.0)
+        else:
+            o.force_fermion_core(x, y, 1, dt, 1.0)
+        if not exp:
+            q.force_clover_logdet(m, 2.0)
+    zero = np.zeros((lat.V, 4, lat.dimg))
+    lat.momenta_set(zero)
+    lat.fermion_force_end_momenta(dt)
+    return lat.momenta_get(), o.fermion_force_end(dt, zero)
+
+
+@pytest.mark.parametrize("exp", [False, True])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 4, 2, 10)])
+@pytest.mark.parametrize("ng,rep", GROUPS)
+def test_clover_force(ng, rep, dims, exp):
+    o, lat, u, _ = setup(ng, dims, rep)
+    got, ref = clover_force_pair(o, lat, exp)
+    # sums of a few hundred products of entries of order one, relative to the largest entry
+    assert np.abs(got - ref).max() < 2e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("uploaded", [False, True])
+def test_clover_force_in_the_representation(uploaded):
+    """Links that are not unitary, and represented links uploaded by themselves."""
+    o, lat, u, _ = setup(3, (4, 2, 2, 4), O.SYM)
+    if uploaded:
+        lat.set_gauge_f(o.represent_gauge_field(u, True))
+    else:
+        u = u * 1.01
+        o.set_gauge(o.represent_gauge_field(u, True))
+        lat.set_gauge(u)
+        lat.represent_gauge_field(True)
+    got, ref = clover_force_pair(o, lat, False)
+    assert np.abs(got - ref).max() < 2e-13 * np.abs(ref).max()
