@@ -151,6 +151,7 @@ int ensure_tmp(void **p, size_t bytes);
 int library_device();  // the device of hrgpu_init (-1 before)
 int ensure_links_bf16();  // the BF16 copy of the links, made from the FP64 ones when they changed
 int detect_recon12();     // check links set already represented for row-2 reconstruction
+void links_flt_written();  // the FP32 copies were made with the FP64 links
 void fund_links_changed(); // the fundamental links were written: stop building represented links from them
 int compute_clover_term_dev();
 void cg_release();

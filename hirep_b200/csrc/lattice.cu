@@ -623,6 +623,13 @@ int ensure_links_bf16() {
 
 }  // namespace hrgpu
 
+namespace hrgpu {
+void links_flt_written() {
+  L.have_gauge_flt = true;
+  L.gauge_gen++;  // every write of the double links ends here
+}
+}  // namespace hrgpu
+
 extern "C" {
 
 int hrgpu_assign_ud2u_f(void) {
@@ -638,8 +645,7 @@ int hrgpu_assign_ud2u_f(void) {
     k_convert<float, double><<<nblk(ng), 256, 0, L.stream>>>((float *)L.Ugf, (const double *)L.Ug, ng);
     HR_LAUNCH_CHECK();
   }
-  L.have_gauge_flt = true;
-  L.gauge_gen++;  // every write of the double links is followed by this call
+  links_flt_written();
   return 0;
 }
 

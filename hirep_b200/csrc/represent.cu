@@ -5,11 +5,80 @@
 //
 // The basis conventions are those of HiRep's explicit formulas, so the
 // represented links agree element by element with the reference's u_gauge_f.
-#include "dirac.cuh"
+#include "suN.cuh"
 
 namespace hrgpu {
 
 constexpr int MAXNG = 8;
+
+// element (C, A) of the represented link of u by HiRep's formulas
+template <int NG, int RP>
+__device__ __forceinline__ double2 rep_elem_exact(const double2 (&u)[NG][NG], int C, int A) {
+  typedef Rep<NG, RP> P;
+  if (RP == HRGPU_FUND) return u[C < NG ? C : 0][A < NG ? A : 0];
+  auto cm = [](double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); };
+  const int c = P::hi(C), e = P::lo(C), a = P::hi(A), b = P::lo(A);
+  if (RP == HRGPU_SYM) {
+    const double st = 1.41421356237309504880, ist = 0.70710678118654752440;
+    const double2 m = a == b ? cm(u[e][a], u[c][a]) : cadd(cm(u[e][a], u[c][b]), cm(u[e][b], u[c][a]));
+    if (e < c) return a == b ? make_double2(st * m.x, st * m.y) : m;
+    return a == b ? m : make_double2(ist * m.x, ist * m.y);
+  }
+  const double2 m = csub(cm(u[e][a], u[c][b]), cm(u[e][b], u[c][a]));
+  return make_double2(-m.x, -m.y);
+}
+
+// The representations up to NG = 4 (NF <= 10, SU(2) adjoint): the link in registers,
+// every element of the represented one a fixed expression (the same products and
+// factors as k_represent), written once in FP64 and, rounded from that value, once
+// in FP32 (assign_ud2u_f's copy, which would read the FP64 links back), with the
+// FP32 fundamental links of the FP32 hop where Ugf is given.  A stream, bound by HBM:
+// NG^2 complex in, NF^2 complex (or real) out in both precisions, 326 MB in 52 us at
+// 16^4 SU(4) antisymmetric (114 us with run-time loops and local memory, and 92 us for
+// the two FP32 copies).
+template <int NG, int RP>
+__global__ void __launch_bounds__(128) k_represent_r(void *Uout, void *Uf, float2 *Ugf, const double2 *Ug, Geo g,
+                                                     int bc_t_anti) {
+  constexpr int NF = Rep<NG, RP>::NF;
+  const long d = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int mu = blockIdx.y;
+  if (d >= 2L * g.ld || (d >= g.ld ? d - g.ld : d) >= g.VH) return;
+  const long lp = 2L * g.ld;
+  const LinkPtr<NG> p = link_at<NG>(Ug, mu, d, lp);
+  double2 u[NG][NG];
+#pragma unroll
+  for (int i = 0; i < NG; i++)
+#pragma unroll
+    for (int j = 0; j < NG; j++) {
+      u[i][j] = p(i, j);
+      if (Ugf) Ugf[((long)mu * NG * NG + i * NG + j) * lp + d] = make_float2((float)u[i][j].x, (float)u[i][j].y);
+    }
+  // time is the slowest coordinate of a parity's sites
+  const long cb = d >= g.ld ? d - g.ld : d;
+  const double sgn = (bc_t_anti && mu == 0 && cb < (long)g.Xh * g.Y * g.Z) ? -1.0 : 1.0;
+  if constexpr (RP == HRGPU_ADJ) {
+    static_assert(NG == 2, "adjoint: SU(2)");
+    double r[3][3];
+    su2_adjoint(r, u);
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const double v = sgn * r[k / 3][k % 3];
+      ((double *)Uout)[((long)mu * 9 + k) * lp + d] = v;
+      ((float *)Uf)[((long)mu * 9 + k) * lp + d] = (float)v;
+    }
+  } else {
+#pragma unroll
+    for (int C = 0; C < NF; C++)
+#pragma unroll
+      for (int A = 0; A < NF; A++) {
+        double2 v = rep_elem_exact<NG, RP>(u, C, A);
+        v = make_double2(sgn * v.x, sgn * v.y);
+        const long e = ((long)mu * NF * NF + C * NF + A) * lp + d;
+        ((double2 *)Uout)[e] = v;
+        ((float2 *)Uf)[e] = make_float2((float)v.x, (float)v.y);
+      }
+  }
+}
 
 // one link: u (NG x NG, complex) -> v (NF x NF) written to the link planes at (mu, d)
 __global__ void k_represent(void *Uout, const double2 *Ug, int ng, int repr, Geo g, int bc_t_anti) {
@@ -238,13 +307,37 @@ int hrgpu_represent_gauge_field(int bc_t_antiperiodic) {
   if (!L.U) HR_CUDA(cudaMalloc(&L.U, (size_t)4 * nel * 2 * L.ld * esz));
   Geo g = make_geo();
   long n = 2L * L.ld;
-  k_represent<<<dim3((unsigned)((n + 127) / 128), 4), 128, 0, L.stream>>>(L.U, L.Ug, L.ng, L.repr, g, bc_t_antiperiodic);
+  const long nflt = (long)4 * nel * 2 * L.ld * (L.real ? 1 : 2);
+  if (!L.Uf) HR_CUDA(cudaMalloc(&L.Uf, nflt * sizeof(float)));
+  const bool two6 = !L.real && L.nf == 6 && ((L.repr == HRGPU_SYM && L.ng == 3) || (L.repr == HRGPU_ASYM && L.ng == 4));
+  if (two6 && !L.Ugf) HR_CUDA(cudaMalloc(&L.Ugf, (size_t)4 * L.ng * L.ng * 2 * L.ld * sizeof(float2)));
+  const dim3 grid((unsigned)((n + 127) / 128), 4);
+  bool flt_done = true;
+#define HR_RP(NGV, RPV) \
+  k_represent_r<NGV, RPV><<<grid, 128, 0, L.stream>>>(L.U, L.Uf, two6 ? L.Ugf : nullptr, L.Ug, g, bc_t_antiperiodic)
+  switch (L.repr * 16 + L.ng) {
+    case HRGPU_FUND * 16 + 2: HR_RP(2, HRGPU_FUND); break;
+    case HRGPU_FUND * 16 + 3: HR_RP(3, HRGPU_FUND); break;
+    case HRGPU_FUND * 16 + 4: HR_RP(4, HRGPU_FUND); break;
+    case HRGPU_ADJ * 16 + 2: HR_RP(2, HRGPU_ADJ); break;
+    case HRGPU_SYM * 16 + 2: HR_RP(2, HRGPU_SYM); break;
+    case HRGPU_SYM * 16 + 3: HR_RP(3, HRGPU_SYM); break;
+    case HRGPU_SYM * 16 + 4: HR_RP(4, HRGPU_SYM); break;
+    case HRGPU_ASYM * 16 + 3: HR_RP(3, HRGPU_ASYM); break;
+    case HRGPU_ASYM * 16 + 4: HR_RP(4, HRGPU_ASYM); break;
+    default:
+      k_represent<<<grid, 128, 0, L.stream>>>(L.U, L.Ug, L.ng, L.repr, g, bc_t_antiperiodic);
+      flt_done = false;
+      break;
+  }
+#undef HR_RP
   HR_LAUNCH_CHECK();
   L.have_gauge = true;
   L.fund_current = true;
   L.bc_t = bc_t_antiperiodic;
   if (int rc = set_recon12(bc_t_antiperiodic, true)) return rc;
-  if (int rc = hrgpu_assign_ud2u_f()) return rc;
+  if (flt_done) links_flt_written();
+  else if (int rc = hrgpu_assign_ud2u_f()) return rc;
   if (L.clover) {
     if (int rc = compute_clover_term_dev()) return rc;
   }

@@ -95,3 +95,32 @@ def test_clover_force_in_the_representation(uploaded):
         lat.represent_gauge_field(True)
     got, ref = clover_force_pair(o, lat, False)
     assert np.abs(got - ref).max() < 2e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 4, 2, 10)])
+@pytest.mark.parametrize("ng,rep", GROUPS + [(5, O.FUND), (4, O.SYM), (3, O.ADJ)])
+def test_links_clover_term_and_inverse(ng, rep, dims):
+    """represent_gauge_field (FP64 and FP32 links), the clover term, D and D^-1 on both parities."""
+    o, lat, u, _ = setup(ng, dims, rep)
+    uf = o.represent_gauge_field(u, True)
+    assert np.abs(lat.gauge_f() - uf).max() < 1e-15 * max(1, o.nf)  # products of two entries of order one
+    o.clover_init(1.3)
+    o.compute_clover_term()
+    lat.clover_init(1.3)
+    # 24 loops of four links
+    assert np.abs(lat.clover_term() - o.clover_term()).max() < 5e-15 * max(1, o.nf)
+    m = 0.2
+    e = F.gaussian_spinor(5, o.V, o.nf)
+    f, out = lat.field(G.FULL, host=e), lat.field(G.FULL)
+    for name in ("Cphi_diag", "Cphi_diag_inv"):
+        getattr(lat, name)(m, out, f)
+        ref = np.concatenate([getattr(o, name)(m, e[p * o.VH:(p + 1) * o.VH], p) for p in range(2)])
+        # the blocks' condition number is below 10
+        assert np.abs(out.download() - ref).max() < 1e-14 * np.abs(ref).max(), name
+    # the FP32 links were made with the FP64 ones
+    lat.Dphi_flt_(lat.field(G.FULL, G.FLOAT), lat.field(G.FULL, G.FLOAT, host=e))
+    o.set_gauge(uf)
+    of = lat.field(G.FULL, G.FLOAT)
+    lat.Dphi_flt_(of, lat.field(G.FULL, G.FLOAT, host=e))
+    ref = o.Dphi_(e, O.FULL, O.FULL)
+    assert np.abs(of.download() - ref).max() < 3e-6 * np.abs(ref).max()
