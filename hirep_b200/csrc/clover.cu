@@ -508,9 +508,13 @@ static int alloc_clover() {
 int compute_clover_term_dev() {
   HR_REQUIRE(L.clover, HRGPU_E_STATE, "compute_clover_term: clover not initialised");
   if (int rc = check_gauge(HRGPU_DOUBLE)) return rc;
-  Geo g = make_geo();
-  HR_NF_DISPATCH(L.real, L.nf, (launch_clover<N_, R_>(L.cl_term, L.U, g, L.csw)));
-  HR_LAUNCH_CHECK();
+  const int rc = clover_term_fund();
+  if (rc > 0) return rc;
+  if (rc < 0) {
+    Geo g = make_geo();
+    HR_NF_DISPATCH(L.real, L.nf, (launch_clover<N_, R_>(L.cl_term, L.U, g, L.csw)));
+    HR_LAUNCH_CHECK();
+  }
   L.sigma = 0xF00F;
   L.sigma_diag = 0xF00F;
   L.sigma_flt = 0xF00F;

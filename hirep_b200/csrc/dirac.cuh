@@ -31,6 +31,7 @@ void batch_release();           // batch.cu: workspaces and captured graphs
 void qmr_release();             // qmr.cu: the g5QMR / MINRES work fields
 void hmc_release();             // hmc.cu: generators, local action
 int fermion_force_finish(double dt);  // force.cu: clover part of fermion_force_end
+int clover_term_fund();  // cterm.cu: the clover term from the fundamental links (-1: not this way)
 int clover_force_fund(double coeff, int **bad);  // cforce.cu: the same through the fundamental links
 
 // clover: make sure the packed (4+m)+A blocks and their inverse exist for this
