@@ -440,50 +440,61 @@ static int force_table_upload() {
   return 0;
 }
 
-// g5 sigma_{mu nu} on a spinor held as [4][N] (force_fermion_core.c:123-250)
-template <int N>
-__device__ __forceinline__ void g5_sigma(double2 (&s)[4][N], const double2 (&u)[4][N], int q) {
-  // q enumerates (0,1),(0,2),(1,2),(0,3),(1,3),(2,3) as cl_force does
-  const int srcs[6][4] = {{1, 0, 3, 2}, {1, 0, 3, 2}, {0, 1, 2, 3}, {0, 1, 2, 3}, {1, 0, 3, 2}, {1, 0, 3, 2}};
-  // factors (re, im)
-  const double fr[6][4] = {{0, 0, 0, 0}, {-1, 1, -1, 1}, {0, 0, 0, 0}, {0, 0, 0, 0}, {-1, 1, 1, -1}, {0, 0, 0, 0}};
-  const double fi[6][4] = {{-1, -1, -1, -1}, {0, 0, 0, 0}, {1, -1, -1, 1}, {-1, 1, -1, 1}, {0, 0, 0, 0}, {1, 1, -1, -1}};
-  for (int c = 0; c < 4; c++)
-    for (int i = 0; i < N; i++) {
-      double2 a = u[srcs[q][c]][i];
-      s[c][i] = make_double2(fr[q][c] * a.x - fi[q][c] * a.y, fr[q][c] * a.y + fi[q][c] * a.x);
-    }
-}
+// g5 sigma_{mu nu} (force_fermion_core.c:123-250) for the six (mu,nu) of cl_force,
+// (0,1),(0,2),(1,2),(0,3),(1,3),(2,3): component c of the result is (fr + i fi)
+// times component src of the input
+__constant__ int c_sig_src[6][4] = {{1, 0, 3, 2}, {1, 0, 3, 2}, {0, 1, 2, 3}, {0, 1, 2, 3}, {1, 0, 3, 2}, {1, 0, 3, 2}};
+__constant__ double c_sig_fr[6][4] = {{0, 0, 0, 0}, {-1, 1, -1, 1}, {0, 0, 0, 0}, {0, 0, 0, 0}, {-1, 1, 1, -1}, {0, 0, 0, 0}};
+__constant__ double c_sig_fi[6][4] = {{-1, -1, -1, -1}, {0, 0, 0, 0}, {1, -1, -1, 1}, {-1, 1, -1, 1}, {0, 0, 0, 0}, {1, 1, -1, -1}};
 
-// force_clover_fermion (force_fermion_core.c:384-454)
+// force_clover_fermion (force_fermion_core.c:384-454): per plane q the matrix
+//   Z_ij = sum_c (sigma Y)_ci conj(X_cj) + (sigma X)_ci conj(Y_cj),
+// anti-Hermitian, so the lower triangle is formed and mirrored.  A block is 32 sites
+// x 6 planes, one warp each; X and Y of the sites are read once into shared memory.
+// acc: add to cl_force, else write it.  Bound by the store (and read) of cl_force,
+// 96 NF^2 bytes per site: 52 us at 24x12^3 SU(3) sextet (280 us with a thread's two
+// spinors and their sigma products in local memory).
 template <int N, bool REAL>
-__global__ void k_force_clover_fermion(double2 *clf, const double2 *X, const double2 *Y, Geo g, double residue) {
-  long d = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  int q = blockIdx.y;
-  if (d >= 2L * g.ld) return;
-  int p = d >= g.ld ? 1 : 0;
-  if (d - p * g.ld >= g.VH) return;
-  double2 xs[4][N], ys[4][N], tl[4][N], tr[4][N];
-  for (int c = 0; c < 4; c++)
-    for (int i = 0; i < N; i++) {
-      xs[c][i] = *sp_at(X, d, c * N + i, g.ld, N);
-      ys[c][i] = *sp_at(Y, d, c * N + i, g.ld, N);
+__global__ void __launch_bounds__(192) k_force_clover_fermion(double2 *clf, const double2 *X, const double2 *Y, Geo g,
+                                                              double residue, int acc) {
+  extern __shared__ double2 fx[];  // [X, Y][4N][32]
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  const long d = (long)blockIdx.x * 32 + lane, lp = 2L * g.ld;
+  const bool on = (d >= g.ld ? d - g.ld : d) < g.VH;
+  for (int c = q; c < 8 * N; c += 6)
+    fx[c * 32 + lane] = on ? __ldg(sp_at(c < 4 * N ? X : Y, d, c < 4 * N ? c : c - 4 * N, g.ld, N)) : make_double2(0.0, 0.0);
+  __syncthreads();
+  if (!on) return;
+  auto xs = [&](int c, int i) { return fx[(c * N + i) * 32 + lane]; };
+  auto ys = [&](int c, int i) { return fx[((4 + c) * N + i) * 32 + lane]; };
+#pragma unroll 1
+  for (int i = 0; i < N; i++) {
+    double2 tl[4], tr[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int src = c_sig_src[q][c];
+      const double fr = residue * c_sig_fr[q][c], fi = residue * c_sig_fi[q][c];
+      const double2 a = ys(src, i), b = xs(src, i);
+      tl[c] = make_double2(fr * a.x - fi * a.y, fr * a.y + fi * a.x);
+      tr[c] = make_double2(fr * b.x - fi * b.y, fr * b.y + fi * b.x);
     }
-  g5_sigma<N>(tr, xs, q);
-  g5_sigma<N>(tl, ys, q);
-  const long lp = 2L * g.ld;
-  for (int i = 0; i < N; i++)
-    for (int j = 0; j < N; j++) {
-      double2 s = make_double2(0, 0);
-      for (int k = 0; k < 4; k++) {
-        cmacc(s, xs[k][j], tl[k][i]);  // tl_i conj(X_j)
-        cmacc(s, ys[k][j], tr[k][i]);  // tr_i conj(Y_j)
+    for (int j = 0; j <= i; j++) {
+      double2 z = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        cmacc(z, xs(c, j), tl[c]);
+        cmacc(z, ys(c, j), tr[c]);
       }
-      if (REAL) s.y = 0.0;
-      double2 &o = clf[((long)q * N * N + i * N + j) * lp + d];
-      o.x += residue * s.x;
-      o.y += residue * s.y;
+      if (REAL) z.y = 0.0;
+      double2 *o = clf + ((long)q * N * N + i * N + j) * lp + d;
+      if (acc) z = cadd(z, *o);
+      *o = z;
+      if (j < i) {
+        // the mirrored element of what is held is -conj of this one's as well
+        clf[((long)q * N * N + j * N + i) * lp + d] = make_double2(-z.x, z.y);
+      }
     }
+  }
 }
 
 // The exponential clover's force matrices (force_fermion_core.c:484-772).  With
@@ -500,11 +511,6 @@ __global__ void k_force_clover_fermion(double2 *clf, const double2 *X, const dou
 // e <- e e.  One block of (2NF)^2 threads per site, one matrix element each,
 // seven 2NF x 2NF matrices in dynamic shared memory.
 constexpr int EXPF_TAYLOR = 16;
-// g5 sigma_{mu nu} for the six (mu,nu) of cl_force: component c of the result is
-// (fr + i fi) times component src of the input (the tables of g5_sigma above)
-__constant__ int c_sig_src[6][4] = {{1, 0, 3, 2}, {1, 0, 3, 2}, {0, 1, 2, 3}, {0, 1, 2, 3}, {1, 0, 3, 2}, {1, 0, 3, 2}};
-__constant__ double c_sig_fr[6][4] = {{0, 0, 0, 0}, {-1, 1, -1, 1}, {0, 0, 0, 0}, {0, 0, 0, 0}, {-1, 1, 1, -1}, {0, 0, 0, 0}};
-__constant__ double c_sig_fi[6][4] = {{-1, -1, -1, -1}, {0, 0, 0, 0}, {1, -1, -1, 1}, {-1, 1, -1, 1}, {0, 0, 0, 0}, {1, 1, -1, -1}};
 template <int N>
 constexpr size_t expf_smem() { return sizeof(double2) * 7 * (2 * N) * (2 * N); }
 
@@ -704,7 +710,9 @@ __global__ void k_force_clover_core(double *fsum, const void *U, const double2 *
 // _compute_clover_force (clover_tools.c:208-298) on odd sites from the packed inverse
 template <int N, bool REAL>
 __global__ void k_force_logdet(double2 *clf, const double *idg, const double2 *iod, Geo g, double coeff) {
-  int cb = blockIdx.x * blockDim.x + threadIdx.x;
+  // 32 sites per block, the elements of the matrices over its warps: 42 us at 24x12^3
+  // SU(3) sextet, 158 us with a thread walking over a site's elements
+  const int cb = blockIdx.x * 32 + (threadIdx.x & 31);
   if (cb >= g.VH) return;
   const long lp = 2L * g.ld, d = (long)g.ld + cb;  // odd sites
   const int n = 2 * N, no = N * (2 * N - 1);
@@ -718,9 +726,8 @@ __global__ void k_force_logdet(double2 *clf, const double *idg, const double2 *i
     }
     return make_double2(coeff * v.x, coeff * v.y);
   };
-  for (int i = 0; i < N; i++)
-    for (int j = 0; j < N; j++) {
-      int ij = i * N + j;
+  for (int ij = threadIdx.x >> 5; ij < N * N; ij += blockDim.x >> 5) {
+      const int i = ij / N, j = ij % N;
       double2 a21 = Ael(0, i + N, j), a12c = Ael(0, j + N, i), a43 = Ael(1, i + N, j), a34c = Ael(1, j + N, i);
       double2 a12 = make_double2(a12c.x, -a12c.y), a34 = make_double2(a34c.x, -a34c.y);
       // the inverse is Hermitian, so conj(A[j][i]) = A[i][j] on both branches of the reference
@@ -831,6 +838,27 @@ static void launch_force_w(double *fsum, const void *U, const double2 *X, const 
   }
 }
 
+template <int N, bool REAL>
+static int launch_clover_fermion(const double2 *X, const double2 *Y, Geo g, double residue) {
+  constexpr int smem = (int)sizeof(double2) * 8 * N * 32;
+  if (smem > 48 * 1024)
+    HR_CUDA(cudaFuncSetAttribute(k_force_clover_fermion<N, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_force_clover_fermion<N, REAL><<<(unsigned)(2L * g.ld / 32), 192, smem, L.stream>>>(L.cl_force, X, Y, g, residue,
+                                                                                   !L.cl_force_zero);
+  L.cl_force_zero = false;
+  return 0;
+}
+
+// cl_force cleared by fermion_force_begin and not written since: its zeros are
+// written here, for whoever adds to it or reads it (the first clover force of an
+// accumulation writes it instead and needs none)
+static int clear_cl_force() {
+  if (!L.cl_force_zero) return 0;
+  HR_CUDA(cudaMemsetAsync(L.cl_force, 0, sizeof(double2) * 6 * L.nf * L.nf * 2 * L.ld, L.stream));
+  L.cl_force_zero = false;
+  return 0;
+}
+
 static ProjTab proj() {
   ProjTab P;
   P.off = L.d_proj_off;
@@ -859,6 +887,7 @@ namespace hrgpu {
 int fermion_force_finish(double dt) {
   if (!L.clover) return 0;
   if (int rc = check_gauge(HRGPU_DOUBLE)) return rc;
+  if (int rc = clear_cl_force()) return rc;
   const double coeff = dt * (L.repr_norm2 / L.fund_norm2) * (1. / 8.) * L.csw;
   Geo g = make_geo();
   const long n = 2L * L.ld;
@@ -879,8 +908,7 @@ int hrgpu_fermion_force_begin(void) {
   HR_REQUIRE(L.ready, HRGPU_E_STATE, "fermion_force_begin: lattice not initialised");
   if (int rc = ensure_force()) return rc;
   HR_CUDA(cudaMemsetAsync(L.force_sum, 0, sizeof(double) * 4 * L.dimg * 2 * L.ld, L.stream));
-  if (L.clover && L.cl_force)
-    HR_CUDA(cudaMemsetAsync(L.cl_force, 0, sizeof(double2) * 6 * L.nf * L.nf * 2 * L.ld, L.stream));
+  L.cl_force_zero = L.clover && L.cl_force;
   return 0;
 }
 
@@ -909,9 +937,10 @@ int hrgpu_force_fermion_core(void *Xs, void *Ys, int auto_fill_odd, double dt, d
   Geo g = make_geo();
   const long n = 2L * L.ld;
   if (L.clover && L.expclover) {
+    if (int rc = clear_cl_force()) return rc;
     HR_NF_DISPATCH(L.real, L.nf, (launch_force_expclover<N_, R_>(L.cl_force, L.cl_term, X, Y, g, 4.0 + static_mass(), residue)));
   } else if (L.clover) {
-    HR_NF_DISPATCH(L.real, L.nf, (k_force_clover_fermion<N_, R_><<<dim3(nb(n), 6), 128, 0, L.stream>>>(L.cl_force, X, Y, g, residue)));
+    HR_NF_DISPATCH(L.real, L.nf, if (int rc = (launch_clover_fermion<N_, R_>(X, Y, g, residue))) return rc);
     HR_LAUNCH_CHECK();
   }
   if ((!L.real && L.nf <= 6) || (L.real && L.nf == 3)) {
@@ -944,8 +973,9 @@ int hrgpu_force_clover_logdet(double mass, double residue) {
   // WITH_CLOVER only, force_fermion_core.c:776-782)
   if (L.expclover) return 0;
   if (int rc = clover_prepare(mass, HRGPU_DOUBLE)) return rc;
+  if (int rc = clear_cl_force()) return rc;
   Geo g = make_geo();
-  HR_NF_DISPATCH(L.real, L.nf, (k_force_logdet<N_, R_><<<nb(L.VH), 128, 0, L.stream>>>(L.cl_force, L.cl_idg, L.cl_iod, g, residue)));
+  HR_NF_DISPATCH(L.real, L.nf, (k_force_logdet<N_, R_><<<nb(L.VH, 32), 384, 0, L.stream>>>(L.cl_force, L.cl_idg, L.cl_iod, g, residue)));
   HR_LAUNCH_CHECK();
   return 0;
 }
@@ -968,6 +998,7 @@ int hrgpu_fermion_force_end(double dt, double *force_host) {
 int hrgpu_clover_force_get(void *host) {
   HR_REQUIRE(L.ready && L.clover && L.cl_force, HRGPU_E_STATE, "clover_force_get: no clover force accumulated");
   HR_REQUIRE(host, HRGPU_E_ARG, "clover_force_get: NULL output");
+  if (int rc = clear_cl_force()) return rc;
   return links_out(host, L.cl_force, L.nf * L.nf, 16, 6);
 }
 

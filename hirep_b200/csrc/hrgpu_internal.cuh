@@ -71,6 +71,7 @@ struct Lattice {
   // clover
   bool clover = false;
   bool expclover = false;         // WITH_EXPCLOVER: diagonal (4+m) exp(A/(4+m))
+  bool cl_force_zero = false;     // cl_force stands for zeros that are not written yet (force.cu)
   double csw = 0.0;
   double sigma = 0xF00F;          // mass term (4+m) the inverse was built for
   double2 *cl_term = nullptr;     // A blocks s0..s3 [4][nf*nf][2*ld]
