@@ -271,33 +271,44 @@ static dim3 bgrid(long rows, int nb) {
   return dim3((unsigned)b, (unsigned)ntiles(nb));
 }
 
-// row of a tile holding component c of site n
-__device__ __forceinline__ long tile_row(long n, long c, int ncomp) {
-  return ((n / TILE_S) * ncomp + c) * TILE_S + (n % TILE_S);
+// separate single-field arrays (element (c, n) at c*ld + n) into a batch, and back.
+// A warp moves one component of 32 sites of a tile: four runs of 8 sites x 4 fields on
+// the batch's side, four fields' runs of 32 sites on the other, through 128 elements
+// of shared memory, so that both sides are whole runs (with one element per thread in
+// single-field order the batch's side was runs of one element, and the index took a
+// 64-bit division per element).
+constexpr int BP_WARPS = 8;
+
+template <typename V, bool PACK>
+__global__ void __launch_bounds__(32 * BP_WARPS) k_bmove(V *batch, V *const *field, int ld, int ncomp, int nb) {
+  __shared__ V sm[BP_WARPS][4 * 33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, tile = blockIdx.y;
+  const long ngroup = ld / 32, item = (long)blockIdx.x * BP_WARPS + w;
+  if (item >= ngroup * ncomp) return;
+  const long group = item / ncomp;
+  const int c = (int)(item - group * ncomp);
+  V *bt = batch + ((((long)tile * (ld / TILE_S) + group * 4) * ncomp + c) * TILE_S) * TILE_F + lane;
+  const long step = (long)ncomp * TILE_S * TILE_F;  // to the next block of 8 sites
+  const int nf = nb - tile * TILE_F < TILE_F ? nb - tile * TILE_F : TILE_F;
+  const long off = (long)c * ld + group * 32 + lane;
+  V *s = sm[w];
+  if (PACK) {
+    for (int f = 0; f < nf; f++) s[(lane >> 3) * 33 + (lane & 7) * TILE_F + f] = field[tile * TILE_F + f][off];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if ((lane & (TILE_F - 1)) < nf) bt[k * step] = s[k * 33 + lane];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) s[k * 33 + lane] = bt[k * step];
+    __syncwarp();
+    for (int f = 0; f < nf; f++) field[tile * TILE_F + f][off] = s[(lane >> 3) * 33 + (lane & 7) * TILE_F + f];
+  }
 }
 
-// separate single-field arrays (element (c, n) at c*ld + n) into a batch, and
-// back; threads run over the single-field order, whose runs of 8 sites are
-// runs of 8 rows of the tile
-template <typename V>
-__global__ void k_bpack(V *dst, const V *const *src, long rows, int ld, int ncomp, int nb) {
-  BMap m = bmap(nb);
-  if (!m.on) return;
-  const V *s = src[m.f];
-  for (long i = m.row; i < rows; i += m.stride) {
-    const long c = i / ld, n = i - c * ld;
-    dst[bix(tile_row(n, c, ncomp), m.f, rows)] = s[i];
-  }
-}
-template <typename V>
-__global__ void k_bunpack(V *const *dst, const V *src, long rows, int ld, int ncomp, int nb) {
-  BMap m = bmap(nb);
-  if (!m.on) return;
-  V *d = dst[m.f];
-  for (long i = m.row; i < rows; i += m.stride) {
-    const long c = i / ld, n = i - c * ld;
-    d[i] = src[bix(tile_row(n, c, ncomp), m.f, rows)];
-  }
+static dim3 bmove_grid(int nb) {
+  const long items = (long)(L.ld / 32) * 4 * L.nf;
+  return dim3((unsigned)((items + BP_WARPS - 1) / BP_WARPS), (unsigned)ntiles(nb));
 }
 
 // per-field Re <a_f, b_f> partials
@@ -856,12 +867,11 @@ int hrgpu_batch_pack(void *batch, const void *const *fields, int nb, int prec) {
              "batch_pack: bad arguments (nb = %d, 1..%d supported)", nb, BMAXS);
   for (int f = 0; f < nb; f++) HR_REQUIRE(fields[f] != nullptr, HRGPU_E_ARG, "batch_pack: field %d is NULL", f);
   if (int rc = bouter_init()) return rc;
-  const long rows = (long)4 * L.nf * L.ld;
   HR_CUDA(cudaMemcpyAsync(BO.d_ptrs, fields, sizeof(void *) * nb, cudaMemcpyHostToDevice, L.stream));
   if (prec == HRGPU_DOUBLE)
-    k_bpack<double2><<<bgrid(rows, nb), BTHREADS, 0, L.stream>>>((double2 *)batch, (const double2 *const *)BO.d_ptrs, rows, L.ld, 4 * L.nf, nb);
+    k_bmove<double2, true><<<bmove_grid(nb), 32 * BP_WARPS, 0, L.stream>>>((double2 *)batch, (double2 *const *)BO.d_ptrs, L.ld, 4 * L.nf, nb);
   else
-    k_bpack<float2><<<bgrid(rows, nb), BTHREADS, 0, L.stream>>>((float2 *)batch, (const float2 *const *)BO.d_ptrs, rows, L.ld, 4 * L.nf, nb);
+    k_bmove<float2, true><<<bmove_grid(nb), 32 * BP_WARPS, 0, L.stream>>>((float2 *)batch, (float2 *const *)BO.d_ptrs, L.ld, 4 * L.nf, nb);
   HR_LAUNCH_CHECK();
   // the pointer array is reused by the next call: finish reading it first
   HR_CUDA(cudaStreamSynchronize(L.stream));
@@ -874,12 +884,11 @@ int hrgpu_batch_unpack(void *const *fields, const void *batch, int nb, int prec)
              "batch_unpack: bad arguments (nb = %d, 1..%d supported)", nb, BMAXS);
   for (int f = 0; f < nb; f++) HR_REQUIRE(fields[f] != nullptr, HRGPU_E_ARG, "batch_unpack: field %d is NULL", f);
   if (int rc = bouter_init()) return rc;
-  const long rows = (long)4 * L.nf * L.ld;
   HR_CUDA(cudaMemcpyAsync(BO.d_ptrs, fields, sizeof(void *) * nb, cudaMemcpyHostToDevice, L.stream));
   if (prec == HRGPU_DOUBLE)
-    k_bunpack<double2><<<bgrid(rows, nb), BTHREADS, 0, L.stream>>>((double2 *const *)BO.d_ptrs, (const double2 *)batch, rows, L.ld, 4 * L.nf, nb);
+    k_bmove<double2, false><<<bmove_grid(nb), 32 * BP_WARPS, 0, L.stream>>>((double2 *)batch, (double2 *const *)BO.d_ptrs, L.ld, 4 * L.nf, nb);
   else
-    k_bunpack<float2><<<bgrid(rows, nb), BTHREADS, 0, L.stream>>>((float2 *const *)BO.d_ptrs, (const float2 *)batch, rows, L.ld, 4 * L.nf, nb);
+    k_bmove<float2, false><<<bmove_grid(nb), 32 * BP_WARPS, 0, L.stream>>>((float2 *)batch, (float2 *const *)BO.d_ptrs, L.ld, 4 * L.nf, nb);
   HR_LAUNCH_CHECK();
   HR_CUDA(cudaStreamSynchronize(L.stream));
   return 0;
