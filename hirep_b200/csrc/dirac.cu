@@ -1,6 +1,7 @@
 // dirac.cu -- Wilson / clover Dirac operators on the device (LibHR/Update/Dphi.c,
 // Dphi_flt.c, D_update.c), built from the fused hopping kernel in hop.cuh.
 #include "dirac.cuh"
+#include "hop_dir.cuh"
 
 namespace hrgpu {
 
@@ -25,14 +26,11 @@ static const void *links() {
   return L.flt_links == HRGPU_LINKS_BF16 ? L.Ubf : L.Uf;
 }
 
-// one hop onto parity outp with the given epilogue; fields are parity fields
 template <typename R>
-int hop(int outp, void *out, const void *in, int ep, double cacc, const void *aux, double caux, int g5, double *red,
-        const R *cdg, const typename C2<R>::T *cod, int cb0, int cb1) {
-  HopArgs<R> a;
+static int hop_args(HopArgs<R> &a, int outp, void *out, const void *in, double cacc, const void *aux, double caux, int g5,
+                    double *red, const R *cdg, const typename C2<R>::T *cod, int cb0, int cb1, const HopTail *tail) {
   a.cb0 = cb0;
-  a.cb1 = cb1 < 0 ? (int)L.VH : cb1;
-  if (a.cb1 <= a.cb0) return 0;
+  a.cb1 = cb1;
   a.in = in;
   a.out = out;
   a.U = links<R>();
@@ -46,38 +44,67 @@ int hop(int outp, void *out, const void *in, int ep, double cacc, const void *au
   a.g5 = g5;
   a.stop = L.cur_stop;
   a.err = nullptr;
+  a.both = 0;
+  a.pre = tail ? tail->pre : 0;
+  a.racc = tail ? tail->racc : nullptr;
+  a.omega = tail ? tail->omega : nullptr;
+  a.red_g5 = tail ? tail->red_g5 : 0;
+  a.no_pdl = tail ? tail->no_pdl : 0;
   a.Ug = sizeof(R) == 8 ? (const void *)L.Ug : (const void *)L.Ugf;
   if (sizeof(R) == 4 && L.flt_links == HRGPU_LINKS_BF16) {
     if (int rc = ensure_links_bf16()) return rc;
     a.U = L.Ubf;
   }
-  if (a.cb0 == 0 && a.cb1 == (int)L.VH) g_mvm++;  // partial launches are counted by their caller
+  return 0;
+}
+
+// one hop onto parity outp with the given epilogue; fields are parity fields
+template <typename R>
+int hop(int outp, void *out, const void *in, int ep, double cacc, const void *aux, double caux, int g5, double *red,
+        const R *cdg, const typename C2<R>::T *cod, int cb0, int cb1, const HopTail *tail) {
+  HopArgs<R> a;
+  if (cb1 < 0) cb1 = (int)L.VH;
+  if (cb1 <= cb0) return 0;
+  if (int rc = hop_args<R>(a, outp, out, in, cacc, aux, caux, g5, red, cdg, cod, cb0, cb1, tail)) return rc;
+  if (cb0 == 0 && cb1 == (int)L.VH) g_mvm++;  // partial launches are counted by their caller
   return launch_hop<R>(ep, a);
 }
 template int hop<double>(int, void *, const void *, int, double, const void *, double, int, double *, const double *,
-                         const double2 *, int, int);
+                         const double2 *, int, int, const HopTail *);
 template int hop<float>(int, void *, const void *, int, double, const void *, double, int, double *, const float *,
-                        const float2 *, int, int);
+                        const float2 *, int, int, const HopTail *);
+
+static int last_hop_variant(int ep, int prec) {
+  const int pi = prec == HRGPU_DOUBLE ? 0 : (L.flt_links == HRGPU_LINKS_BF16 ? 2 : 1);
+  return L.hop_force >= 0 ? L.hop_force : L.hop_variant[pi][ep];
+}
+
+// the hop onto both parities of a full field: one launch where the variant in use
+// takes both (a small lattice then fills twice the SMs), else one per parity
+template <typename R>
+static int hop_full(void *out, const void *in, int ep, double cacc, const void *aux, double caux, int g5, const R *cdg,
+                    const typename C2<R>::T *cod) {
+  const int v = last_hop_variant(ep, sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT);
+  const size_t half = (size_t)4 * L.nf * L.ld * sizeof(typename C2<R>::T);
+  if (v == 1 && L.nf <= 6) {
+    HopArgs<R> a;
+    if (int rc = hop_args<R>(a, HRGPU_EVEN, out, in, cacc, aux, caux, g5, nullptr, cdg, cod, 0, (int)L.VH, nullptr)) return rc;
+    a.both = 1;
+    g_mvm += 2;
+    return launch_hop<R>(ep, a);
+  }
+  for (int p = 0; p < 2; p++)
+    if (int rc = hop<R>(p, (char *)out + p * half, (const char *)in + (p ^ 1) * half, ep, cacc,
+                        aux ? (const char *)aux + p * half : nullptr, caux, g5, nullptr, cdg, cod))
+      return rc;
+  return 0;
+}
 
 int check_gauge(int prec) {
   HR_REQUIRE(L.ready, HRGPU_E_STATE, "lattice not initialised");
   if (prec == HRGPU_DOUBLE) HR_REQUIRE(L.have_gauge, HRGPU_E_STATE, "no gauge field set");
   else HR_REQUIRE(L.have_gauge_flt, HRGPU_E_STATE, "no float gauge field set");
   return 0;
-}
-
-template <typename R>
-static size_t par_elems() {
-  return (size_t)4 * L.nf * L.ld;  // complex elements of one parity field
-}
-
-template <typename R>
-static inline void *par_ptr(void *f, int p) {
-  return (char *)f + (size_t)p * par_elems<R>() * sizeof(typename C2<R>::T);
-}
-template <typename R>
-static inline const void *par_ptr(const void *f, int p) {
-  return (const char *)f + (size_t)p * par_elems<R>() * sizeof(typename C2<R>::T);
 }
 
 // Dphi_ on parity or full fields
@@ -87,10 +114,7 @@ int Dphi_hop(void *out, int out_par, const void *in) {
   HR_REQUIRE(out && in && out != in, HRGPU_E_ARG, "Dphi_: input and output fields must be different");
   HR_REQUIRE(out_par >= 0 && out_par <= 2, HRGPU_E_ARG, "Dphi_: bad parity");
   if (out_par == HRGPU_FULL) {
-    for (int p = 0; p < 2; p++)
-      if (int rc = hop<R>(p, par_ptr<R>(out, p), par_ptr<R>(in, p ^ 1), EP_AXPY, -0.5, nullptr, 0.0, 0, nullptr,
-                          nullptr, nullptr))
-        return rc;
+    if (int rc = hop_full<R>(out, in, EP_AXPY, -0.5, nullptr, 0.0, 0, nullptr, nullptr)) return rc;
     g_mvm++;  // a full-lattice application counts twice (Dphi.c:205-207)
     return 0;
   }
@@ -102,11 +126,7 @@ template <typename R>
 int Dphi_full(double m0, void *out, const void *in, int g5) {
   if (int rc = check_gauge(sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT)) return rc;
   HR_REQUIRE(out && in && out != in, HRGPU_E_ARG, "Dphi: input and output fields must be different");
-  for (int p = 0; p < 2; p++)
-    if (int rc = hop<R>(p, par_ptr<R>(out, p), par_ptr<R>(in, p ^ 1), EP_AXPY, -0.5, par_ptr<R>(in, p), 4.0 + m0, g5,
-                        nullptr, nullptr, nullptr))
-      return rc;
-  return 0;
+  return hop_full<R>(out, in, EP_AXPY, -0.5, in, 4.0 + m0, g5, nullptr, nullptr);
 }
 
 // one hop of an even-odd preconditioned operator with output parity p, on the
@@ -118,15 +138,21 @@ int Dphi_full(double m0, void *out, const void *in, int g5) {
 // further in every direction).
 template <typename R>
 int eo_stage(int clover, double mass, int stage, int outp, void *out, const void *in, int g5, double *red, int cb0,
-             int cb1) {
+             int cb1, const HopTail *tail) {
   void **tmp = sizeof(R) == 8 ? &L.tmp_o : &L.tmp_o_f;
   if (int rc = ensure_tmp(tmp, spinor_bytes(HRGPU_EVEN, sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT))) return rc;
+  // the second hop follows the first, which has waited for whatever made the links,
+  // the clover blocks and in
+  HopTail ht;
+  if (tail) ht = *tail;
+  ht.pre = 1;
+  tail = stage ? &ht : nullptr;
   if (clover) {
     const R *idg, *ddg;
     const typename C2<R>::T *iod, *dod;
     clover_blocks<R>(&ddg, &dod, &idg, &iod);
     if (stage == 0) return hop<R>(outp ^ 1, *tmp, in, EP_CLOV_INV, -0.5, nullptr, 0.0, 0, nullptr, idg, iod, cb0, cb1);
-    return hop<R>(outp, out, *tmp, EP_CLOV, 0.5, in, 0.0, g5, red, ddg, dod, cb0, cb1);
+    return hop<R>(outp, out, *tmp, EP_CLOV, 0.5, in, 0.0, g5, red, ddg, dod, cb0, cb1, tail);
   }
   if (stage == 0) return hop<R>(outp ^ 1, *tmp, in, EP_AXPY, -0.5, nullptr, 0.0, 0, nullptr, nullptr, nullptr, cb0, cb1);
   double rho = 4.0 + mass;
@@ -136,35 +162,35 @@ int eo_stage(int clover, double mass, int stage, int outp, void *out, const void
   } else {
     rho = rho * rho;
   }
-  return hop<R>(outp, out, *tmp, EP_AXPY, 0.5, in, rho, g5, red, nullptr, nullptr, cb0, cb1);
+  return hop<R>(outp, out, *tmp, EP_AXPY, 0.5, in, rho, g5, red, nullptr, nullptr, cb0, cb1, tail);
 }
-template int eo_stage<double>(int, double, int, int, void *, const void *, int, double *, int, int);
-template int eo_stage<float>(int, double, int, int, void *, const void *, int, double *, int, int);
+template int eo_stage<double>(int, double, int, int, void *, const void *, int, double *, int, int, const HopTail *);
+template int eo_stage<float>(int, double, int, int, void *, const void *, int, double *, int, int, const HopTail *);
 
 // even-odd: out = (4+m)^2 in - D_pq D_qp in on parity p, optionally gamma_5
 template <typename R>
-int Dphi_eo(double m0, void *out, const void *in, int outp, int g5, double *red) {
+int Dphi_eo(double m0, void *out, const void *in, int outp, int g5, double *red, const HopTail *tail) {
   if (int rc = check_gauge(sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT)) return rc;
   HR_REQUIRE(out && in && out != in, HRGPU_E_ARG, "Dphi_eopre: input and output fields must be different");
   if (int rc = eo_stage<R>(0, m0, 0, outp, out, in, g5, nullptr, 0, -1)) return rc;
-  return eo_stage<R>(0, m0, 1, outp, out, in, g5, red, 0, -1);
+  return eo_stage<R>(0, m0, 1, outp, out, in, g5, red, 0, -1, tail);
 }
 
-template int Dphi_eo<double>(double, void *, const void *, int, int, double *);
-template int Dphi_eo<float>(double, void *, const void *, int, int, double *);
+template int Dphi_eo<double>(double, void *, const void *, int, int, double *, const HopTail *);
+template int Dphi_eo<float>(double, void *, const void *, int, int, double *, const HopTail *);
 
 // ------------------------------------------------------------------ clover
 template <typename R>
-int Cphi_eo(double mass, void *out, const void *in, int g5, double *red) {
+int Cphi_eo(double mass, void *out, const void *in, int g5, double *red, const HopTail *tail) {
   if (int rc = check_gauge(sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT)) return rc;
   HR_REQUIRE(L.clover, HRGPU_E_STATE, "Cphi_eopre: no clover term (hrgpu_clover_init)");
   HR_REQUIRE(out && in && out != in, HRGPU_E_ARG, "Cphi_eopre: input and output fields must be different");
   if (int rc = clover_prepare(mass, sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT)) return rc;
   if (int rc = eo_stage<R>(1, mass, 0, HRGPU_EVEN, out, in, g5, nullptr, 0, -1)) return rc;
-  return eo_stage<R>(1, mass, 1, HRGPU_EVEN, out, in, g5, red, 0, -1);
+  return eo_stage<R>(1, mass, 1, HRGPU_EVEN, out, in, g5, red, 0, -1, tail);
 }
-template int Cphi_eo<double>(double, void *, const void *, int, double *);
-template int Cphi_eo<float>(double, void *, const void *, int, double *);
+template int Cphi_eo<double>(double, void *, const void *, int, double *, const HopTail *);
+template int Cphi_eo<float>(double, void *, const void *, int, double *, const HopTail *);
 
 static int Cphi_full(double mass, void *out, const void *in, int g5) {
   if (int rc = check_gauge(HRGPU_DOUBLE)) return rc;
@@ -174,11 +200,7 @@ static int Cphi_full(double mass, void *out, const void *in, int g5) {
   const double *idg, *ddg;
   const double2 *iod, *dod;
   clover_blocks<double>(&ddg, &dod, &idg, &iod);
-  for (int p = 0; p < 2; p++)
-    if (int rc = hop<double>(p, par_ptr<double>(out, p), par_ptr<double>(in, p ^ 1), EP_CLOV, -0.5,
-                             par_ptr<double>(in, p), 0.0, g5, nullptr, ddg, dod))
-      return rc;
-  return 0;
+  return hop_full<double>(out, in, EP_CLOV, -0.5, in, 0.0, g5, ddg, dod);
 }
 
 template <typename R>
@@ -224,31 +246,41 @@ int apply_op(int op, int prec, double mass, void *out, const void *in) {
   return HRGPU_E_ARG;
 }
 
-// The even-odd H^2 (op G5DPHI_EOPRE_SQ or G5CPHI_EOPRE_SQ), the same launches
-// as apply_op, with the |H in|^2 partial sums of the first H application (one
-// per block of its last hop) in red[0 .. *nblocks): with H Hermitian,
-// <in, H^2 in> = |H in|^2, the CG's alpha without a dot-product pass.
-// Returns -1 when op has no such form (the caller takes the dot product), else
-// 0 or an error status.
-template <typename R>
-static int sq_eo_sqnorm(bool clover, double m, void *out, const void *in, double *red, int *nblocks) {
-  void **tmp = sizeof(R) == 8 ? &L.tmp_e : &L.tmp_e_f;
-  if (int rc = ensure_tmp(tmp, spinor_bytes(HRGPU_EVEN, sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT))) return rc;
-  if (int rc = clover ? Cphi_eo<R>(m, *tmp, in, 1, red) : Dphi_eo<R>(m, *tmp, in, HRGPU_EVEN, 1, red)) return rc;
-  // the block count of the variant that ran (tuned now if it was the first launch)
-  const int pi = sizeof(R) == 8 ? 0 : (L.flt_links == HRGPU_LINKS_BF16 ? 2 : 1);
-  const int ep = clover ? EP_CLOV : EP_AXPY;
-  const int v = L.hop_force >= 0 ? L.hop_force : L.hop_variant[pi][ep];
-  const long threads = hop_threads_per_site(v) * (long)L.VH;
-  *nblocks = (int)((threads + HOP_THREADS - 1) / HOP_THREADS);
-  return clover ? Cphi_eo<R>(m, out, *tmp, 1, nullptr) : Dphi_eo<R>(m, out, *tmp, HRGPU_EVEN, 1, nullptr);
+int hop_red_blocks(bool clover, int prec) {
+  int v = last_hop_variant(clover ? EP_CLOV : EP_AXPY, prec);
+  if (v == 6 && L.hop_force < 0 && (L.recon12 < 3 || !L.recon_allow)) v = 0;  // what the launcher then runs
+  return v < 0 ? 0 : hop_blocks(v, L.VH, L.nf);
 }
 
+bool hop_tail_settled(bool clover, int prec) {
+  const int v = last_hop_variant(clover ? EP_CLOV : EP_AXPY, prec);
+  return v >= 0 && hop_tail_ok(v, L.nf, prec == HRGPU_FLOAT && L.flt_links == HRGPU_LINKS_BF16);
+}
+
+int apply_eo(bool clover, int prec, double mass, void *out, const void *in, int g5, double *red, const HopTail *tail) {
+  if (prec == HRGPU_DOUBLE)
+    return clover ? Cphi_eo<double>(mass, out, in, g5, red, tail) : Dphi_eo<double>(mass, out, in, HRGPU_EVEN, g5, red, tail);
+  return clover ? Cphi_eo<float>(mass, out, in, g5, red, tail) : Dphi_eo<float>(mass, out, in, HRGPU_EVEN, g5, red, tail);
+}
+
+// The even-odd H^2 (op G5DPHI_EOPRE_SQ or G5CPHI_EOPRE_SQ) with the |H in|^2 partial
+// sums of the first H application: with H Hermitian, <in, H^2 in> = |H in|^2, the
+// CG's alpha without a dot-product pass.  -1 when op has no such form.
 int apply_op_sqnorm(int op, int prec, double mass, void *out, const void *in, double *red, int *nblocks) {
   if (op != HRGPU_OP_G5DPHI_EOPRE_SQ && op != HRGPU_OP_G5CPHI_EOPRE_SQ) return -1;
   const bool clover = op == HRGPU_OP_G5CPHI_EOPRE_SQ;
-  return prec == HRGPU_DOUBLE ? sq_eo_sqnorm<double>(clover, mass, out, in, red, nblocks)
-                              : sq_eo_sqnorm<float>(clover, mass, out, in, red, nblocks);
+  void *tmp = eo_tmp(prec);
+  if (!tmp) return HRGPU_E_CUDA;
+  if (int rc = apply_eo(clover, prec, mass, tmp, in, 1, red, nullptr)) return rc;
+  *nblocks = hop_red_blocks(clover, prec);
+  return apply_eo(clover, prec, mass, out, tmp, 1, nullptr, nullptr);
+}
+
+bool hop_small(bool clover, int prec) { return L.nf <= 6 && last_hop_variant(clover ? EP_CLOV : EP_AXPY, prec) == 1; }
+
+void *eo_tmp(int prec) {
+  void **tmp = prec == HRGPU_DOUBLE ? &L.tmp_e : &L.tmp_e_f;
+  return ensure_tmp(tmp, spinor_bytes(HRGPU_EVEN, prec)) ? nullptr : *tmp;
 }
 
 int op_parity(int op) {

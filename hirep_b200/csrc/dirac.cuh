@@ -10,19 +10,41 @@ int launch_hop(int ep, HopArgs<R> &a);
 
 template <typename R>
 int hop(int outp, void *out, const void *in, int ep, double cacc, const void *aux, double caux, int g5, double *red,
-        const R *cdg, const typename C2<R>::T *cod, int cb0 = 0, int cb1 = -1);
+        const R *cdg, const typename C2<R>::T *cod, int cb0 = 0, int cb1 = -1, const HopTail *tail = nullptr);
 
 int check_gauge(int prec);
 template <typename R>
 int eo_stage(int clover, double mass, int stage, int outp, void *out, const void *in, int g5, double *red, int cb0,
-             int cb1);
+             int cb1, const HopTail *tail = nullptr);
 template <typename R>
-int Dphi_eo(double m0, void *out, const void *in, int outp, int g5, double *red);
+int Dphi_eo(double m0, void *out, const void *in, int outp, int g5, double *red, const HopTail *tail = nullptr);
 template <typename R>
-int Cphi_eo(double mass, void *out, const void *in, int g5, double *red);
+int Cphi_eo(double mass, void *out, const void *in, int g5, double *red, const HopTail *tail = nullptr);
 int apply_op(int op, int prec, double mass, void *out, const void *in);
 int apply_op_sqnorm(int op, int prec, double mass, void *out, const void *in, double *red, int *nblocks);
+// one application D (H: gamma_5 D) of an even-odd operator with the |out|^2 (or
+// tail's) partial sums of its last hop in red[0 .. hop_red_blocks(...))
+int apply_eo(bool clover, int prec, double mass, void *out, const void *in, int g5, double *red, const HopTail *tail);
+int hop_red_blocks(bool clover, int prec);  // of the variant in use; 0 while it is not tuned
+bool hop_tail_settled(bool clover, int prec);  // the variant in use is tuned and has the inverters' forms
+bool hop_small(bool clover, int prec);  // the variant in use is the one for small lattices
+void *eo_tmp(int prec);  // the even temporary of the squared operators (nullptr on failure, message set)
 int op_parity(int op);
+
+// a kernel that begins with pdl_enter(), launched to overlap the end of the one before it (pdl) or plainly
+template <typename... A, typename... B>
+static inline cudaError_t launch_after(bool pdl, void (*f)(A...), unsigned grid, unsigned block, B... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = L.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, f, (A)args...);
+}
 double static_mass();
 void add_mvm(unsigned long n);  // hops done outside hop(), e.g. replayed CUDA graphs
 unsigned long mvm_count();      // the raw hop counter (captures read and restore it)

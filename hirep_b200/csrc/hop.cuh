@@ -43,7 +43,22 @@ struct HopArgs {
   int cb0, cb1;      // output sites cb0 <= cb < cb1 of parity outp
   int recon;         // Lattice::recon12 at launch: 2 (4) puts the antiperiodic sign on rebuilt rows (links)
   const void *Ug;    // fundamental links [4][NG*NG][2ld], element type of R (two-index links built on the fly, recon 3, 4)
+  int both;          // k_hop_dir: both parities of full fields in one launch (outp is not used)
+  int pre;           // the launch before this one is a hop of the same operator: what no hop writes
+                     // (links, clover blocks, aux) may be read before waiting for it (k_hop_dir)
+  // second hop of an operator inside an inverter (hop_tail_ok's variants):
+  void *racc;           // non-null: racc += *omega * result instead of out = result, red is of the new racc
+  const double *omega;
+  int no_pdl;           // a launch that joins two branches of a graph
+  int red_g5;           // red is Re <gamma_5 aux, result> instead of |result|^2
   Geo g;
+};
+
+// the inverters' forms of an operator's last hop (see HopArgs)
+struct HopTail {
+  void *racc = nullptr;
+  const double *omega = nullptr;
+  int red_g5 = 0, no_pdl = 0, pre = 0;
 };
 
 template <bool REAL, typename R>
@@ -497,8 +512,10 @@ __device__ __forceinline__ void two_idx_mul2(V *c0, V *c1, const V *h0, const V 
 // element of component 0, components HOP_THREADS apart) once the bulk copies on
 // the mbarrier at shared address bar have landed; the t direction is then
 // visited last, after x, y, z, to give the copies time
+// TAIL: the inverters' forms (HopArgs::racc, red_g5), compiled apart because the code
+// costs the plain epilogue 3 % (FP32 adjoint at 64x32^3)
 template <int NFT, bool REAL, typename R, int EP, typename LE = typename LinkE<REAL, R>::T, bool TSM = false,
-          bool RC = false, int FR = 0>
+          bool RC = false, int FR = 0, bool TAIL = false>
 __device__ __forceinline__ double hop_site(const HopArgs<R> &a, const int cb, const typename C2<R>::T *tsu = nullptr,
                                            const typename C2<R>::T *tsd = nullptr, unsigned bar = 0) {
   typedef typename C2<R>::T V;
@@ -627,6 +644,24 @@ __device__ __forceinline__ double hop_site(const HopArgs<R> &a, const int cb, co
       clover_epilogue<NA, EP>(r2, r3, a, ca, cb, 1, cb, ld);
     }
     const R sg = a.g5 ? (R)-1 : (R)1;
+    if (TAIL && a.racc) {
+      const R om = (R)*a.omega;
+      V *rp = (V *)a.racc + cb;
+      auto acc = [&](int c, V v) {
+        V r = rp[(long)c * ld];
+        rmac(r, om, v);
+        rp[(long)c * ld] = r;
+        nrm += (double)r.x * r.x + (double)r.y * r.y;
+      };
+#pragma unroll
+      for (int i = 0; i < NA; i++) {
+        acc(i, r0[i]);
+        acc(nf + i, r1[i]);
+        acc(2 * nf + i, cscale(sg, r2[i]));
+        acc(3 * nf + i, cscale(sg, r3[i]));
+      }
+      return nrm;
+    }
 #pragma unroll
     for (int i = 0; i < NA; i++) {
       if (i >= nf) break;
@@ -635,7 +670,14 @@ __device__ __forceinline__ double hop_site(const HopArgs<R> &a, const int cb, co
       out[(long)(1 * nf + i) * ld] = r1[i];
       out[(long)(2 * nf + i) * ld] = o2;
       out[(long)(3 * nf + i) * ld] = o3;
-      if (a.red) {
+      if (TAIL && a.red_g5) {
+        const V *ax = (const V *)a.aux + cb;
+        auto dot = [&](int c, V v) {
+          const V u = ld_c(ax + (long)c * ld);
+          return (double)u.x * v.x + (double)u.y * v.y;
+        };
+        nrm += dot(i, r0[i]) + dot(nf + i, r1[i]) - dot(2 * nf + i, o2) - dot(3 * nf + i, o3);
+      } else if (a.red) {
         nrm += (double)r0[i].x * r0[i].x + (double)r0[i].y * r0[i].y + (double)r1[i].x * r1[i].x +
                (double)r1[i].y * r1[i].y + (double)o2.x * o2.x + (double)o2.y * o2.y + (double)o3.x * o3.x +
                (double)o3.y * o3.y;
@@ -645,30 +687,29 @@ __device__ __forceinline__ double hop_site(const HopArgs<R> &a, const int cb, co
   return nrm;
 }
 
-// threads per output site of a single-field hop variant: 2 for the spin-split
-// variants 1 and 3, 1 for the others (0, 2, 4 and 5)
-__host__ __device__ constexpr int hop_threads_per_site(int variant) { return (variant == 1 || variant == 3) ? 2 : 1; }
-
 // Programmatic dependent launch: let the next kernel of the stream be scheduled
 // as soon as every block of this one has started (its blocks then fill the SMs
 // that this launch's last, partial wave leaves idle), and wait for the previous
 // kernel and its memory before touching global memory.  Both are no-ops for a
 // launch without the programmatic-serialization attribute.
+// The dependents are let go after the wait, so that whatever ran before this launch is
+// complete and visible when the next kernel starts (k_hop_dir reads before its wait).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
+  pdl_wait();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // RC: rebuild row 2 of the 3x3 links (instantiated for NF = 3 only); FR: build
 // the NF = 6 two-index links from the fundamental ones (see TwoIdx)
 template <int NFT, bool REAL, typename R, int EP, int MINB, typename LE = typename LinkE<REAL, R>::T, bool RC = false,
-          int FR = 0>
+          int FR = 0, bool TAIL = false>
 __global__ void __launch_bounds__(HOP_THREADS, MINB) k_hop(HopArgs<R> a) {
   pdl_enter();
   if (a.stop && *a.stop) return;
   const int cb = a.cb0 + blockIdx.x * blockDim.x + threadIdx.x;
   double nrm = 0.0;
-  if (cb < a.cb1) nrm = hop_site<NFT, REAL, R, EP, LE, false, RC, FR>(a, cb);
+  if (cb < a.cb1) nrm = hop_site<NFT, REAL, R, EP, LE, false, RC, FR, TAIL>(a, cb);
   if (a.red) block_partial<R>(nrm, a.red);
 }
 

@@ -4,6 +4,7 @@
 #pragma once
 #include "dirac.cuh"
 #include "hop_async.cuh"
+#include "hop_dir.cuh"
 #include "hop_tma.cuh"
 
 namespace hrgpu {
@@ -18,7 +19,7 @@ namespace hrgpu {
 // that the copy-stream kernels beside them needed: 0.47 -> 0.69 ms).
 template <typename R>
 static inline cudaError_t launch_pdl(void (*kernel)(HopArgs<R>), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                     HopArgs<R> &a) {
+                                     HopArgs<R> &a, bool small = false) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -28,7 +29,7 @@ static inline cudaError_t launch_pdl(void (*kernel)(HopArgs<R>), dim3 grid, dim3
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = (L.hop_pdl && sizeof(R) == 8 && a.cb0 == 0 && a.cb1 == (int)L.VH) ? 1 : 0;
+  cfg.numAttrs = (L.hop_pdl && !a.no_pdl && (sizeof(R) == 8 || small) && a.cb0 == 0 && a.cb1 == (int)L.VH) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
@@ -72,11 +73,39 @@ int launch_tma(HopArgs<R> &a, dim3 grid, dim3 block, cudaStream_t s) {
 // 3x3 links (SU(3) fundamental, SU(2) adjoint) when the links passed the
 // check, else the one reading full links
 template <int N, bool RL, typename R, int EP, int MINB>
-static inline void (*hop_kernel(int recon))(HopArgs<R>) {
+static inline void (*hop_kernel(int recon, bool tail))(HopArgs<R>) {
+  typedef typename LinkE<RL, R>::T LE;
+  constexpr bool T = EP != EP_CLOV_INV;  // the first hop of a clover operator has no inverters' form
   if constexpr (N == 3) {
-    if (recon) return k_hop<N, RL, R, EP, MINB, typename LinkE<RL, R>::T, true>;
+    if (recon) return tail ? k_hop<N, RL, R, EP, MINB, LE, true, 0, T> : k_hop<N, RL, R, EP, MINB, LE, true>;
   }
-  return k_hop<N, RL, R, EP, MINB>;
+  return tail ? k_hop<N, RL, R, EP, MINB, LE, false, 0, T> : k_hop<N, RL, R, EP, MINB>;
+}
+
+// variant 1: one warp per direction (k_hop_dir) for NF <= 6, two threads per site
+// (k_hop2) for larger NF.  Links are rebuilt or built from the fundamental ones where
+// variants 0 and 6 would do so.
+template <int N, bool RL, typename R, int EP, typename LE = typename LinkE<RL, R>::T>
+int launch_dir(HopArgs<R> &a, long nsites, cudaStream_t s) {
+  if constexpr (HopDirOK<N>::v) {
+    constexpr bool stored = std::is_same<LE, typename LinkE<RL, R>::T>::value;  // not BF16
+    void (*f)(HopArgs<R>) = k_hop_dir<N, RL, R, EP, 2, LE>;
+    if constexpr (stored && N == 3) {
+      if (a.recon) f = k_hop_dir<N, RL, R, EP, 2, LE, true>;
+    }
+    if constexpr (stored && N == 6 && !RL) {
+      if (a.recon >= 3 && a.Ug) f = L.repr == HRGPU_SYM ? k_hop_dir<N, RL, R, EP, 2, LE, false, 1> : k_hop_dir<N, RL, R, EP, 2, LE, false, 2>;
+    }
+    constexpr int smem = HopDirLayout<N, R, EP>::SMEM;
+    if (smem > 40 * 1024)  // with the static part of the norm's sum, at NF = 6
+      HR_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const dim3 grid((unsigned)((nsites + HD_SITES - 1) / HD_SITES), a.both ? 2 : 1);
+    HR_CUDA(launch_pdl<R>(f, grid, dim3(HD_THREADS), smem, s, a, true));
+  } else {
+    const dim3 grid((unsigned)((2 * nsites + HOP_THREADS - 1) / HOP_THREADS));
+    HR_CUDA(launch_pdl<R>(k_hop2<N, RL, R, EP, 1, LE>, grid, dim3(HOP_THREADS), 0, s, a));
+  }
+  return 0;
 }
 
 // variant 6: k_hop (variant 0's register budget) building the NF = 6
@@ -87,10 +116,13 @@ template <int N, bool RL, typename R, int EP>
 int launch_fund(HopArgs<R> &a, dim3 grid, dim3 block, cudaStream_t s) {
   if constexpr (N == 6 && !RL) {
     if (a.recon < 3 || !a.Ug) return -1;
-    if (L.repr == HRGPU_SYM)
-      HR_CUDA(launch_pdl<R>(k_hop<N, RL, R, EP, 1, typename LinkE<RL, R>::T, false, 1>, grid, block, 0, s, a));
-    else
-      HR_CUDA(launch_pdl<R>(k_hop<N, RL, R, EP, 1, typename LinkE<RL, R>::T, false, 2>, grid, block, 0, s, a));
+    typedef typename LinkE<RL, R>::T LE;
+    constexpr bool T = EP != EP_CLOV_INV;
+    const bool tail = a.racc || a.red_g5;
+    void (*f)(HopArgs<R>);
+    if (L.repr == HRGPU_SYM) f = tail ? k_hop<N, RL, R, EP, 1, LE, false, 1, T> : k_hop<N, RL, R, EP, 1, LE, false, 1>;
+    else f = tail ? k_hop<N, RL, R, EP, 1, LE, false, 2, T> : k_hop<N, RL, R, EP, 1, LE, false, 2>;
+    HR_CUDA(launch_pdl<R>(f, grid, block, 0, s, a));
     return 0;
   } else {
     return -1;
@@ -102,22 +134,26 @@ int launch_ep_variant(HopArgs<R> &a, int variant) {
   a.g = make_geo();
   a.nf = L.nf;
   a.recon = L.recon_allow ? L.recon12 : 0;
-  // variants: 0 one thread per site, 1 two threads per site (spin split),
-  // 2 and 3 the same with the register budget capped for 4 resident blocks per SM,
+  // variants: 0 one thread per site, 1 one warp per direction (NF <= 6; else two threads
+  // per site, spin split), 2 as 0 and 3 the spin split with the register budget capped
+  // for 4 resident blocks per SM,
   // 4 one thread per site with the per-direction loads pipelined through shared memory,
   // 5 one thread per site with the time halo staged by bulk (TMA) copies,
   // 6 one thread per site building the NF = 6 two-index links from the fundamental ones
   const long nsites = a.cb1 - a.cb0;
-  const long threads = hop_threads_per_site(variant) * nsites;
-  dim3 grid((unsigned)((threads + HOP_THREADS - 1) / HOP_THREADS)), block(HOP_THREADS);
+  dim3 grid((unsigned)((nsites + HOP_THREADS - 1) / HOP_THREADS)), block(HOP_THREADS);
+  dim3 grid2((unsigned)((2 * nsites + HOP_THREADS - 1) / HOP_THREADS));
+  const bool tail = a.racc || a.red_g5;
   cudaStream_t s = L.stream;
 #define HOPV(N, RL)                                                                    \
   case N:                                                                              \
     switch (variant) {                                                                 \
-      case 0: HR_CUDA(launch_pdl<R>(hop_kernel<N, RL, R, EP, 1>(a.recon), grid, block, 0, s, a)); break; \
-      case 1: HR_CUDA(launch_pdl<R>(k_hop2<N, RL, R, EP, 1>, grid, block, 0, s, a)); break; \
-      case 2: HR_CUDA(launch_pdl<R>(hop_kernel<N, RL, R, EP, 4>(a.recon), grid, block, 0, s, a)); break; \
-      case 3: HR_CUDA(launch_pdl<R>(k_hop2<N, RL, R, EP, 4>, grid, block, 0, s, a)); break; \
+      case 0: HR_CUDA(launch_pdl<R>(hop_kernel<N, RL, R, EP, 1>(a.recon, tail), grid, block, 0, s, a)); break; \
+      case 1:                                                                          \
+        if (int rc_ = launch_dir<N, RL, R, EP>(a, nsites, s)) return rc_;              \
+        break;                                                                         \
+      case 3: HR_CUDA(launch_pdl<R>(k_hop2<N, RL, R, EP, 4>, grid2, block, 0, s, a)); break; \
+      case 2: HR_CUDA(launch_pdl<R>(hop_kernel<N, RL, R, EP, 4>(a.recon, tail), grid, block, 0, s, a)); break; \
       case 4:                                                                          \
         if (int rc_ = launch_async<N, RL, R, EP>(a, grid, block, s)) return rc_;       \
         break;                                                                         \
@@ -136,9 +172,11 @@ int launch_ep_variant(HopArgs<R> &a, int variant) {
   case N:                                                                                       \
     switch (variant) {                                                                          \
       case 0: HR_CUDA(launch_pdl<float>(k_hop<N, RL, float, EP, 1, typename LinkBF16<RL>::T>, grid, block, 0, s, a)); break;  \
-      case 1: HR_CUDA(launch_pdl<float>(k_hop2<N, RL, float, EP, 1, typename LinkBF16<RL>::T>, grid, block, 0, s, a)); break; \
+      case 1:                                                                                   \
+        if (int rc_ = launch_dir<N, RL, float, EP, typename LinkBF16<RL>::T>(a, nsites, s)) return rc_; \
+        break;                                                                                  \
+      case 3: HR_CUDA(launch_pdl<float>(k_hop2<N, RL, float, EP, 4, typename LinkBF16<RL>::T>, grid2, block, 0, s, a)); break; \
       case 2: HR_CUDA(launch_pdl<float>(k_hop<N, RL, float, EP, 4, typename LinkBF16<RL>::T>, grid, block, 0, s, a)); break;  \
-      case 3: HR_CUDA(launch_pdl<float>(k_hop2<N, RL, float, EP, 4, typename LinkBF16<RL>::T>, grid, block, 0, s, a)); break; \
       default: return -1;                                                                       \
     }                                                                                           \
     break;
@@ -229,9 +267,10 @@ int launch_ep(HopArgs<R> &a) {
     }
     return rc;
   }
-  if (v < 0 && (a.cb0 != 0 || a.cb1 != L.VH)) {
-    // a launch over part of the lattice is no measure for the full operator:
-    // run the default variant and leave tuning to the first full launch
+  if (v < 0 && (a.cb0 != 0 || a.cb1 != L.VH || a.racc)) {
+    // a launch over part of the lattice is no measure for the full operator, and
+    // one that accumulates cannot be repeated: run the default variant and leave
+    // tuning to the first full launch
     return launch_ep_variant<R, EP>(a, 0);
   }
   if (v < 0) {

@@ -157,8 +157,9 @@ int hrgpu_g5Dphi_sq_flt(double m0, void *out, const void *in);
 int hrgpu_Dphi_eopre_flt(double m0, void *out, const void *in);
 int hrgpu_g5Dphi_eopre_flt(double m0, void *out, const void *in);
 int hrgpu_g5Dphi_eopre_sq_flt(double m0, void *out, const void *in);
-/* Hopping-kernel variant: 0 = one thread per site, 1 = two threads per site
- * (spin split), 2 and 3 = the same with registers capped for 4 blocks per SM,
+/* Hopping-kernel variant: 0 = one thread per site, 1 = one warp per direction on 32
+ * sites (NF <= 6; larger NF two threads per site, spin split), 2 = as 0 and 3 = spin
+ * split with registers capped for 4 blocks per SM,
  * 4 = one thread per site with cp.async-pipelined loads, 5 = one thread per site
  * with the time halo staged in shared memory by bulk (TMA) copies (4 and 5: NF <= 4
  * complex, NF = 3 real; 5 also needs time slabs of a multiple of 128 sites per
