@@ -4,15 +4,18 @@
 // The recursion is HiRep's, term for term, but every scalar (alpha, omega,
 // gamma, delta and the per-shift z1/z2/z3 and flags) lives in device memory and
 // is updated by one-block "fold" kernels, so an iteration never waits for the
-// host.  One iteration is
-//   M k (the fused hopping kernels) -> <k,Mk> partials -> fold_alpha ->
-//   update1 (x_i += c_i p_i, r += omega Mk, |r|^2 partials) -> fold_lambda ->
-//   update2 (k = gamma k + r, p_i = d_i p_i + z3_i r) -> advance
-// The host launches several iterations at a time (a captured CUDA graph) and
-// reads one state word between chunks.  When fold_lambda finds the stopping condition it marks the
+// host.  One iteration with the even-odd H^2 is
+//   H k (two hops, the last with the |H k|^2 = <k, H^2 k> partials) ->
+//   fold_alpha, beside the first hop of the second H -> its last hop, which adds
+//   omega H^2 k to r instead of writing it and leaves the |r|^2 partials ->
+//   fold_lambda -> update (k = gamma k + r, x_i += c_i p_i, p_i = d_i p_i + z3_i r)
+// With another operator the products and r += omega M k are kernels of their own.
+// The host launches several iterations at a time (a captured CUDA graph), one chunk
+// ahead of the state that it reads.  When fold_lambda finds the stopping condition it marks the
 // state; the remaining kernels of that iteration finish it exactly as HiRep's
 // loop body would, and every kernel of later iterations returns at once, so the
 // solution and the iteration count are those of HiRep's loop.
+#include <type_traits>
 #include <vector>
 
 #include "dirac.cuh"
@@ -31,63 +34,87 @@ struct CGState {
   int flag[MAXS];
 };
 
-__device__ double fold_partials(const double *partials, int nblocks, int stride, int off) {
+constexpr int FOLD_THREADS = 512;
+
+// sum of the partials in a fixed order, eight loads in flight per thread
+__device__ double fold_partials(const double *partials, int nblocks, int stride) {
   double s = 0;
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += partials[(long)b * stride + off];
+  int b = threadIdx.x;
+  for (; b + 7 * (int)blockDim.x < nblocks; b += 8 * blockDim.x) {
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = partials[(long)(b + k * (int)blockDim.x) * stride];
+#pragma unroll
+    for (int k = 0; k < 8; k++) s += v[k];
+  }
+  for (; b < nblocks; b += blockDim.x) s += partials[(long)b * stride];
   return block_sum(s);
 }
 
-// alpha = <k, Mk>; omega = -delta/alpha; z3 and the solution coefficients (cg_mshift.c:82-91)
-__global__ void k_cg_fold_alpha(CGState *S, const double *partials, int nblocks, int stride) {
-  if (S->state != 0) return;
-  double alpha = fold_partials(partials, nblocks, stride, 0);
-  if (threadIdx.x == 0) {
-    S->alpha = alpha;
-    if (!isfinite(alpha) || alpha == 0.0) {  // breakdown (non-positive operator or NaN input)
-      S->state = 3;
-      return;
+// alpha = <k, Mk>; omega = -delta/alpha; z3 and the solution coefficients
+// (cg_mshift.c:82-91), one thread per shift.  The first kernel of an iteration to
+// change the state: an iteration after the one that converged only marks the end.
+__global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_alpha(CGState *S, const double *partials, int nblocks, int stride) {
+  if (S->state != 0) {
+    if (threadIdx.x == 0 && S->state == 1) S->state = 2;
+    return;
+  }
+  const double alpha = fold_partials(partials, nblocks, stride);
+  const bool bad = !isfinite(alpha) || alpha == 0.0;  // breakdown (non-positive operator or NaN input)
+  const double omega = -S->delta / alpha, oldomega = S->omega, gamma = S->gamma;
+  const int i = threadIdx.x;
+  if (!bad && i < S->n) {
+    if (S->flag[i]) {
+      const double z1 = S->z1[i], z2 = S->z2[i];
+      const double z3 = oldomega * z1 * z2 / (omega * gamma * (z1 - z2) + z1 * oldomega * (1. + S->shift[i] * omega));
+      S->z3[i] = z3;
+      S->cx[i] = -omega * z3 / z2;
+    } else {
+      S->cx[i] = 0.0;
     }
-    S->oldomega = S->omega;
-    S->omega = -S->delta / alpha;
-    double omega = S->omega, oldomega = S->oldomega, gamma = S->gamma;
-    for (int i = 0; i < S->n; i++) {
-      if (S->flag[i]) {
-        double z1 = S->z1[i], z2 = S->z2[i];
-        double z3 = oldomega * z1 * z2 / (omega * gamma * (z1 - z2) + z1 * oldomega * (1. + S->shift[i] * omega));
-        S->z3[i] = z3;
-        S->cx[i] = -omega * z3 / z2;
-      } else {
-        S->cx[i] = 0.0;
-      }
+  }
+  __syncthreads();
+  if (i == 0) {
+    S->alpha = alpha;
+    if (bad) {
+      S->state = 3;
+    } else {
+      S->oldomega = oldomega;
+      S->omega = omega;
     }
   }
 }
 
 // lambda = |r|^2, gamma, convergence flags (cg_mshift.c:92-111; cg_mshift_flt.c:96-118)
-__global__ void k_cg_fold_lambda(CGState *S, const double *partials, int nblocks) {
+__global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_lambda(CGState *S, const double *partials, int nblocks) {
+  pdl_enter();
   if (S->state != 0) return;
-  double lambda = fold_partials(partials, nblocks, 1, 0);
-  if (threadIdx.x == 0) {
-    S->lambda = lambda;
-    S->gamma = lambda / S->delta;
-    S->delta = lambda;
-    double gamma = S->gamma, delta = S->delta;
-    int notconv = 0;
-    for (int i = 0; i < S->n; i++) {
-      double z3 = S->z3[i];
-      if (S->flt) {
-        if (delta * z3 * z3 > S->err2 * S->innorm2) ++notconv;
-      } else {
-        if (delta * z3 * z3 < S->err2 * S->innorm2) S->flag[i] = 0;
-        if (S->flag[i]) ++notconv;
-      }
-      if (S->flag[i]) {
-        double z2 = S->z2[i];
-        S->cp[i] = gamma * z3 * z3 / (z2 * z2);
-        S->z1[i] = S->z2[i];
-        S->z2[i] = z3;
-      }
+  const double lambda = fold_partials(partials, nblocks, 1);
+  const double gamma = lambda / S->delta;
+  const int i = threadIdx.x;
+  int open = 0;
+  if (i < S->n) {
+    const double z3 = S->z3[i], lim = S->err2 * S->innorm2;
+    int flag = S->flag[i];
+    if (S->flt) {
+      open = lambda * z3 * z3 > lim;
+    } else {
+      if (lambda * z3 * z3 < lim) S->flag[i] = flag = 0;
+      open = flag;
     }
+    // a shift that converged in this iteration keeps its z's, and gets its last x in the update
+    if (flag) {
+      const double z2 = S->z2[i];
+      S->cp[i] = gamma * z3 * z3 / (z2 * z2);
+      S->z1[i] = z2;
+      S->z2[i] = z3;
+    }
+  }
+  const int notconv = __syncthreads_count(open);
+  if (i == 0) {
+    S->lambda = lambda;
+    S->gamma = gamma;
+    S->delta = lambda;
     S->notconv = notconv;
     S->iter++;
     if (!isfinite(lambda)) S->state = 3;
@@ -95,25 +122,14 @@ __global__ void k_cg_fold_lambda(CGState *S, const double *partials, int nblocks
   }
 }
 
-__global__ void k_cg_advance(CGState *S) {
-  if (S->state == 1) S->state = 2;
-}
-
+// r += omega Mk with |r|^2 partials, for the operators whose last hop does not do it
 template <typename V>
-__global__ void __launch_bounds__(RED_THREADS) k_cg_update1(CGState *S, V *const *x, V *const *p, V *r, const V *Mk,
-                                                            long n, double *partials) {
+__global__ void __launch_bounds__(RED_THREADS) k_cg_update_r(CGState *S, V *r, const V *Mk, long n, double *partials) {
   if (S->state != 0) return;
   const double omega = S->omega;
-  const int ns = S->n;
   double nrm = 0.0;
   long stride = (long)gridDim.x * blockDim.x;
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    for (int i = 0; i < ns; i++) {
-      if (!S->flag[i]) continue;
-      V xv = x[i][e];
-      rmac(xv, (decltype(xv.x))S->cx[i], p[i][e]);
-      x[i][e] = xv;
-    }
     V rv = r[e];
     rmac(rv, (decltype(rv.x))omega, Mk[e]);
     r[e] = rv;
@@ -123,28 +139,53 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_update1(CGState *S, V *const
   if (threadIdx.x == 0) partials[blockIdx.x] = nrm;
 }
 
-template <typename V>
-__global__ void k_cg_update2(CGState *S, V *const *p, V *k, const V *r, long n) {
+// one 16-byte word of a field: one FP64 complex number or two FP32 ones
+__device__ __forceinline__ double2 fma_r(double a, double2 x, double2 y) { return make_double2(fma(a, x.x, y.x), fma(a, x.y, y.y)); }
+__device__ __forceinline__ float4 fma_r(float a, float4 x, float4 y) {
+  return make_float4(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y), fmaf(a, x.z, y.z), fmaf(a, x.w, y.w));
+}
+__device__ __forceinline__ double2 mul_r(double a, double2 x) { return make_double2(a * x.x, a * x.y); }
+__device__ __forceinline__ float4 mul_r(float a, float4 x) { return make_float4(a * x.x, a * x.y, a * x.z, a * x.w); }
+
+// x_i += cx_i p_i and p_i = cp_i p_i + z3_i r for every shift, k = gamma k + r: p_i
+// is read once for both.  one: a single unshifted system, whose p_i is k (every z
+// is 1), so that k serves for both and p_0 is not touched.
+// W: 16-byte words.  (FP32 solves run on the library's own fields only; an FP64
+// complex number is one word, so a caller's field needs no more than its own alignment.)
+template <typename W, typename R, bool PDL>
+__global__ void __launch_bounds__(RED_THREADS) k_cg_update(const CGState *S, W *const *x, W *const *p, W *k, const W *r, long n,
+                                                           int one) {
+  if (PDL) pdl_enter();
   if (S->state >= 2) return;
-  typedef decltype(k[0].x) R;
-  const R gamma = (R)S->gamma;
+  __shared__ R cx[MAXS], cp[MAXS], z3[MAXS];
+  __shared__ int flag[MAXS];
+  __shared__ W *px[MAXS], *pp[MAXS];
   const int ns = S->n;
-  long stride = (long)gridDim.x * blockDim.x;
+  const R gamma = (R)S->gamma;
+  for (int i = threadIdx.x; i < ns; i += blockDim.x) {
+    cx[i] = (R)S->cx[i];
+    cp[i] = (R)S->cp[i];
+    z3[i] = (R)S->z3[i];
+    flag[i] = S->flag[i];
+    px[i] = x[i];
+    pp[i] = p[i];
+  }
+  __syncthreads();
+  const long stride = (long)gridDim.x * blockDim.x;
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    V rv = r[e];
-    V kv = k[e];
-    kv.x = gamma * kv.x + rv.x;
-    kv.y = gamma * kv.y + rv.y;
-    k[e] = kv;
-    for (int i = 0; i < ns; i++) {
-      if (!S->flag[i]) continue;
-      V pv = p[i][e];
-      R cp = (R)S->cp[i], z3 = (R)S->z3[i];
-      pv.x = cp * pv.x;
-      pv.y = cp * pv.y;
-      rmac(pv, z3, rv);
-      p[i][e] = pv;
+    const W rv = r[e], kv = k[e];
+    if (one) {
+      px[0][e] = fma_r(cx[0], kv, px[0][e]);
+    } else {
+#pragma unroll 2
+      for (int i = 0; i < ns; i++) {
+        if (cx[i] == (R)0) continue;
+        const W pv = pp[i][e];
+        px[i][e] = fma_r(cx[i], pv, px[i][e]);
+        if (flag[i]) pp[i][e] = fma_r(z3[i], rv, mul_r(cp[i], pv));
+      }
     }
+    k[e] = fma_r(gamma, kv, rv);
   }
 }
 
@@ -172,7 +213,8 @@ struct CGWork {
   std::vector<void *> bufs;  // p[0..n-1], k, r, Mk
   size_t bytes = 0;
   CGState *S = nullptr;
-  CGState *hS = nullptr;  // pinned host copy
+  CGState *hS = nullptr;  // pinned host copies of the last two chunks' states
+  cudaEvent_t ev[2] = {nullptr, nullptr};
   void **d_ptrs = nullptr;  // device arrays of pointers: x[MAXS], p[MAXS]
 };
 static CGWork W[2];  // [prec]
@@ -199,7 +241,8 @@ static int cg_workspace(int prec, int nvec, size_t bytes) {
   }
   if (!w.S) {
     HR_CUDA(cudaMalloc(&w.S, sizeof(CGState)));
-    HR_CUDA(cudaMallocHost(&w.hS, sizeof(CGState)));
+    HR_CUDA(cudaMallocHost(&w.hS, 2 * sizeof(CGState)));
+    for (cudaEvent_t &ev : w.ev) HR_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     HR_CUDA(cudaMalloc(&w.d_ptrs, sizeof(void *) * 2 * MAXS));
   }
   return 0;
@@ -217,12 +260,13 @@ struct CGGraph {
   int op = -1;
   double mass = 0;
   const void *ptrs[10] = {};
-  int v[3] = {-1, -1, -1}, force = -1, flt_links = -1, pdl = -1;
+  int v[3] = {-1, -1, -1}, force = -1, flt_links = -1, pdl = -1, recon = -1, one = -1;
   unsigned long mvm = 0;  // hop launches in one replay (the MVM counter)
   cudaGraphExec_t exec = nullptr;
 };
 static CGGraph CGG[2];  // [prec]
-static cudaStream_t cg_cap = nullptr;
+static cudaStream_t cg_cap = nullptr, cg_cap2 = nullptr;  // capture streams: the iteration, the fold beside a hop
+static cudaEvent_t cg_ev[2] = {nullptr, nullptr};
 
 static void drop_cg_graph(CGGraph &c) {
   if (c.exec) cudaGraphExecDestroy(c.exec);
@@ -239,13 +283,22 @@ void cg_release() {
   FW = FltWork();
   for (int q = 0; q < 2; q++) drop_cg_graph(CGG[q]);
   if (cg_cap) cudaStreamDestroy(cg_cap);
-  cg_cap = nullptr;
+  if (cg_cap2) cudaStreamDestroy(cg_cap2);
+  for (cudaEvent_t &ev : cg_ev) {
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
+  }
+  cg_cap = cg_cap2 = nullptr;
   for (int q = 0; q < 2; q++) {
     for (void *b : W[q].bufs) cudaFree(b);
     W[q].bufs.clear();
     W[q].bytes = 0;
     if (W[q].S) cudaFree(W[q].S);
     if (W[q].hS) cudaFreeHost(W[q].hS);
+    for (cudaEvent_t &ev : W[q].ev) {
+      if (ev) cudaEventDestroy(ev);
+      ev = nullptr;
+    }
     if (W[q].d_ptrs) cudaFree(W[q].d_ptrs);
     W[q].S = nullptr;
     W[q].hS = nullptr;
@@ -258,29 +311,60 @@ static unsigned red_grid(long n) {
   return (unsigned)(b < RED_MAX_BLOCKS ? b : RED_MAX_BLOCKS);
 }
 
-// CG_CHUNK iterations, launched one kernel at a time
+// CG_CHUNK iterations, launched one kernel at a time.  side: a second stream of the
+// capture in progress for the fold beside a hop, or nullptr.
 template <typename R>
-static int cg_iterations(int op, int prec, double mass, CGWork &w, void *k, void *r, void *Mk, long ne, unsigned g) {
+static int cg_iterations(int op, int prec, double mass, CGWork &w, void *k, void *r, void *Mk, long ne, unsigned g,
+                         int one, cudaStream_t side) {
   typedef typename C2<R>::T V;
-  V *const *dx = (V *const *)w.d_ptrs;
-  V *const *dp = (V *const *)(w.d_ptrs + MAXS);
+  typedef typename std::conditional<sizeof(R) == 8, double2, float4>::type W;
+  const long nw = ne * (long)sizeof(V) / (long)sizeof(W);
+  W *const *dx = (W *const *)w.d_ptrs;
+  W *const *dp = (W *const *)(w.d_ptrs + MAXS);
+  const bool eo = op == HRGPU_OP_G5DPHI_EOPRE_SQ || op == HRGPU_OP_G5CPHI_EOPRE_SQ;
+  const bool clover = op == HRGPU_OP_G5CPHI_EOPRE_SQ;
+  const bool small = eo && L.hop_pdl && hop_small(clover, prec);
+  double *part2 = L.partials + L.npart / 2;  // |r|^2, while the |Hk|^2 ones may still be read
   for (int c = 0; c < CG_CHUNK; c++) {
-    // alpha = <k, H^2 k> = |H k|^2 from the first H's partials where the
-    // operator is the even-odd H^2, else from a dot-product pass
-    int nb = 0;
-    const int rc = apply_op_sqnorm(op, prec, mass, Mk, k, L.partials, &nb);
-    if (rc > 0) return rc;
-    if (rc == 0) {
-      k_cg_fold_alpha<<<1, RED_THREADS, 0, L.stream>>>(w.S, L.partials, nb, 1);
+    unsigned nlam = g;
+    if (eo) {
+      // alpha = <k, H^2 k> = |H k|^2 from the first H's partials
+      void *tmp = eo_tmp(prec);
+      if (!tmp) return HRGPU_E_CUDA;
+      if (int q = apply_eo(clover, prec, mass, tmp, k, 1, L.partials, nullptr)) return q;
+      const int nb = hop_red_blocks(clover, prec);  // tuned by now
+      const bool tail = hop_tail_settled(clover, prec);
+      cudaStream_t fs = tail && side ? side : L.stream;
+      if (fs != L.stream) {
+        HR_CUDA(cudaEventRecord(cg_ev[0], L.stream));
+        HR_CUDA(cudaStreamWaitEvent(fs, cg_ev[0], 0));
+      }
+      k_cg_fold_alpha<<<1, FOLD_THREADS, 0, fs>>>(w.S, L.partials, nb, 1);
+      if (fs != L.stream) HR_CUDA(cudaEventRecord(cg_ev[1], fs));
+      if (tail) {
+        HopTail t;
+        t.racc = r;
+        t.omega = &w.S->omega;
+        t.no_pdl = fs != L.stream;
+        // the second H, joined by the fold before its last hop
+        if (int q = eo_stage<R>(clover, mass, 0, HRGPU_EVEN, Mk, tmp, 1, nullptr, 0, -1)) return q;
+        if (fs != L.stream) HR_CUDA(cudaStreamWaitEvent(L.stream, cg_ev[1], 0));
+        if (int q = eo_stage<R>(clover, mass, 1, HRGPU_EVEN, Mk, tmp, 1, part2, 0, -1, &t)) return q;
+        nlam = (unsigned)nb;
+      } else {
+        if (int q = apply_eo(clover, prec, mass, Mk, tmp, 1, nullptr, nullptr)) return q;
+        k_cg_update_r<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (V *)r, (const V *)Mk, ne, part2);
+      }
     } else {
       if (int q = apply_op(op, prec, mass, Mk, k)) return q;
       k_cg_dot<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (const V *)k, (const V *)Mk, ne, L.partials);
-      k_cg_fold_alpha<<<1, RED_THREADS, 0, L.stream>>>(w.S, L.partials, g, 2);
+      k_cg_fold_alpha<<<1, FOLD_THREADS, 0, L.stream>>>(w.S, L.partials, g, 2);
+      k_cg_update_r<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (V *)r, (const V *)Mk, ne, part2);
     }
-    k_cg_update1<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, dx, dp, (V *)r, (const V *)Mk, ne, L.partials);
-    k_cg_fold_lambda<<<1, RED_THREADS, 0, L.stream>>>(w.S, L.partials, g);
-    k_cg_update2<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, dp, (V *)k, (const V *)r, ne);
-    k_cg_advance<<<1, 1, 0, L.stream>>>(w.S);
+    // on a small lattice, where the launches count, these start while the kernel before ends
+    const bool pdl = side && small;
+    HR_CUDA(launch_after(pdl, k_cg_fold_lambda, 1u, (unsigned)FOLD_THREADS, w.S, part2, (int)nlam));
+    HR_CUDA(launch_after(pdl, pdl ? k_cg_update<W, R, true> : k_cg_update<W, R, false>, red_grid(nw), (unsigned)RED_THREADS, w.S, dx, dp, (W *)k, (const W *)r, nw, one));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "cg iteration", __FILE__, __LINE__);
   }
@@ -290,8 +374,10 @@ static bool op_is_clover(int op) {
   return op == HRGPU_OP_G5CPHI_EOPRE_SQ || op == HRGPU_OP_G5CPHI_SQ || op == HRGPU_OP_CPHI_EOPRE ||
          op == HRGPU_OP_G5CPHI_EOPRE || op == HRGPU_OP_CPHI;
 }
+// *mvm: the hops of the chunk launched, for the caller to count when it is known that they ran
 template <typename R>
-static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, void *Mk, long ne, unsigned g) {
+static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, void *Mk, long ne, unsigned g, int one,
+                    unsigned long *mvm) {
   if (op_is_clover(op))
     if (int rc = clover_prepare(mass, prec)) return rc;
   if (prec == HRGPU_FLOAT && L.flt_links == HRGPU_LINKS_BF16)
@@ -302,25 +388,36 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, 
                                                       (op == HRGPU_OP_G5CPHI_SQ || op == HRGPU_OP_CPHI ||
                                                        L.hop_variant[pi][EP_CLOV_INV] >= 0))
                                                    : L.hop_variant[pi][EP_AXPY] >= 0);
-  if (!settled) return cg_iterations<R>(op, prec, mass, w, k, r, Mk, ne, g);  // tunes the hopping kernels
+  if (!settled) {  // tunes the hopping kernels
+    const unsigned long m0 = mvm_count();
+    const int rc = cg_iterations<R>(op, prec, mass, w, k, r, Mk, ne, g, one, nullptr);
+    *mvm = mvm_count() - m0;
+    mvm_restore(m0);
+    return rc;
+  }
   const void *links = prec == HRGPU_DOUBLE ? (const void *)L.U
                                            : (L.flt_links == HRGPU_LINKS_BF16 ? (const void *)L.Ubf : (const void *)L.Uf);
   const void *ptrs[10] = {k, r, Mk, w.S, w.d_ptrs, L.partials, links, L.cur_stop,
                           prec == HRGPU_DOUBLE ? L.tmp_e : L.tmp_e_f, prec == HRGPU_DOUBLE ? L.tmp_o : L.tmp_o_f};
   CGGraph &c = CGG[prec];
+  const int recon = L.recon_allow ? L.recon12 : 0;
   bool same = c.exec && c.op == op && c.mass == mass && c.force == L.hop_force && c.flt_links == L.flt_links &&
-              c.pdl == (int)L.hop_pdl;
+              c.pdl == (int)L.hop_pdl && c.recon == recon && c.one == one;
   for (int i = 0; i < 3 && same; i++) same = c.v[i] == L.hop_variant[pi][i];
   for (int i = 0; i < 10 && same; i++) same = c.ptrs[i] == ptrs[i];
   if (!same) {
     drop_cg_graph(c);
-    if (!cg_cap) HR_CUDA(cudaStreamCreateWithFlags(&cg_cap, cudaStreamNonBlocking));
+    if (!cg_cap) {
+      HR_CUDA(cudaStreamCreateWithFlags(&cg_cap, cudaStreamNonBlocking));
+      HR_CUDA(cudaStreamCreateWithFlags(&cg_cap2, cudaStreamNonBlocking));
+      for (cudaEvent_t &ev : cg_ev) HR_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    }
     const unsigned long m0 = mvm_count();
     cudaGraph_t graph = nullptr;
     cudaStream_t saved = L.stream;
     HR_CUDA(cudaStreamBeginCapture(cg_cap, cudaStreamCaptureModeRelaxed));
     L.stream = cg_cap;
-    int rc = cg_iterations<R>(op, prec, mass, w, k, r, Mk, ne, g);
+    int rc = cg_iterations<R>(op, prec, mass, w, k, r, Mk, ne, g, one, cg_cap2);
     L.stream = saved;
     cudaError_t e = cudaStreamEndCapture(cg_cap, &graph);
     const unsigned long dm = mvm_count() - m0;
@@ -341,12 +438,14 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, 
     c.force = L.hop_force;
     c.flt_links = L.flt_links;
     c.pdl = (int)L.hop_pdl;
+    c.recon = recon;
+    c.one = one;
     for (int i = 0; i < 3; i++) c.v[i] = L.hop_variant[pi][i];
     for (int i = 0; i < 10; i++) c.ptrs[i] = ptrs[i];
     c.mvm = dm;
   }
   HR_CUDA(cudaGraphLaunch(c.exec, L.stream));
-  add_mvm(c.mvm);
+  *mvm = c.mvm;
   return 0;
 }
 
@@ -393,25 +492,26 @@ static int cg_core(int op, double mass, int n, const double *shift, double err2,
     HR_CUDA(cudaMemcpyAsync(w.bufs[i], r, bytes, cudaMemcpyDeviceToDevice, L.stream));
     if (n != 1) HR_CUDA(cudaMemsetAsync(out[i], 0, bytes, L.stream));
   }
-  CGState &h = *w.hS;
-  memset(&h, 0, sizeof(CGState));
-  h.omega = 1.0;
-  h.gamma = 0.0;
-  h.delta = delta;
-  h.innorm2 = innorm2;
-  h.err2 = err2;
-  h.n = n;
-  h.state = 0;
-  h.iter = 0;
-  h.max_iter = max_iter == 0 ? CG_HARD_LIMIT : (max_iter > cgiter ? max_iter - cgiter : 1);
-  h.flt = flt;
+  // (la_dot above has waited for the stream, so no copy into hS is in flight)
+  CGState &h0 = w.hS[0];
+  memset(&h0, 0, sizeof(CGState));
+  h0.omega = 1.0;
+  h0.gamma = 0.0;
+  h0.delta = delta;
+  h0.innorm2 = innorm2;
+  h0.err2 = err2;
+  h0.n = n;
+  h0.state = 0;
+  h0.iter = 0;
+  h0.max_iter = max_iter == 0 ? CG_HARD_LIMIT : (max_iter > cgiter ? max_iter - cgiter : 1);
+  h0.flt = flt;
   for (int i = 0; i < n; i++) {
-    h.shift[i] = shift[i];
-    h.z1[i] = h.z2[i] = 1.0;
-    h.z3[i] = 0.0;
-    h.flag[i] = flt ? flags[i] : 1;
+    h0.shift[i] = shift[i];
+    h0.z1[i] = h0.z2[i] = 1.0;
+    h0.z3[i] = 0.0;
+    h0.flag[i] = flt ? flags[i] : 1;
   }
-  HR_CUDA(cudaMemcpyAsync(w.S, &h, sizeof(CGState), cudaMemcpyHostToDevice, L.stream));
+  HR_CUDA(cudaMemcpyAsync(w.S, &h0, sizeof(CGState), cudaMemcpyHostToDevice, L.stream));
   void *ptrs[2 * MAXS];
   for (int i = 0; i < n; i++) {
     ptrs[i] = out[i];
@@ -421,19 +521,33 @@ static int cg_core(int op, double mass, int n, const double *shift, double err2,
   const unsigned g = red_grid(ne);
   L.cur_stop = &w.S->state;
   int rc = 0;
-  for (;;) {
-    rc = cg_chunk<R>(op, prec, mass, w, k, r, Mk, ne, g);
+  // one chunk is in flight behind the one whose state is read; the kernels of a
+  // chunk that follows the last iteration return at once and its hops are not counted
+  const int one = n == 1 && shift[0] == 0.0;
+  unsigned long mvm[2] = {0, 0};
+  auto launch = [&](int b) -> int {
+    if (int q = cg_chunk<R>(op, prec, mass, w, k, r, Mk, ne, g, one, &mvm[b])) return q;
+    HR_CUDA(cudaMemcpyAsync(&w.hS[b], w.S, sizeof(CGState), cudaMemcpyDeviceToHost, L.stream));
+    HR_CUDA(cudaEventRecord(w.ev[b], L.stream));
+    return 0;
+  };
+  rc = launch(0);
+  int cur = 0;
+  while (!rc) {
+    rc = launch(cur ^ 1);
     if (rc) break;
-    cudaError_t e = cudaMemcpyAsync(&h, w.S, sizeof(CGState), cudaMemcpyDeviceToHost, L.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(L.stream);
+    cudaError_t e = cudaEventSynchronize(w.ev[cur]);
     if (e != cudaSuccess) {
       rc = fail_cuda(e, "cg state readback", __FILE__, __LINE__);
       break;
     }
-    if (h.state != 0) break;
+    add_mvm(mvm[cur]);
+    if (w.hS[cur].state != 0) break;
+    cur ^= 1;
   }
   L.cur_stop = nullptr;
   if (rc) return rc;
+  const CGState &h = w.hS[cur];
   cgiter += h.iter;
   if (h.state == 3) {
     *iters = cgiter;

@@ -263,19 +263,6 @@ int apply_eo(bool clover, int prec, double mass, void *out, const void *in, int 
   return clover ? Cphi_eo<float>(mass, out, in, g5, red, tail) : Dphi_eo<float>(mass, out, in, HRGPU_EVEN, g5, red, tail);
 }
 
-// The even-odd H^2 (op G5DPHI_EOPRE_SQ or G5CPHI_EOPRE_SQ) with the |H in|^2 partial
-// sums of the first H application: with H Hermitian, <in, H^2 in> = |H in|^2, the
-// CG's alpha without a dot-product pass.  -1 when op has no such form.
-int apply_op_sqnorm(int op, int prec, double mass, void *out, const void *in, double *red, int *nblocks) {
-  if (op != HRGPU_OP_G5DPHI_EOPRE_SQ && op != HRGPU_OP_G5CPHI_EOPRE_SQ) return -1;
-  const bool clover = op == HRGPU_OP_G5CPHI_EOPRE_SQ;
-  void *tmp = eo_tmp(prec);
-  if (!tmp) return HRGPU_E_CUDA;
-  if (int rc = apply_eo(clover, prec, mass, tmp, in, 1, red, nullptr)) return rc;
-  *nblocks = hop_red_blocks(clover, prec);
-  return apply_eo(clover, prec, mass, out, tmp, 1, nullptr, nullptr);
-}
-
 bool hop_small(bool clover, int prec) { return L.nf <= 6 && last_hop_variant(clover ? EP_CLOV : EP_AXPY, prec) == 1; }
 
 void *eo_tmp(int prec) {

@@ -21,7 +21,6 @@ int Dphi_eo(double m0, void *out, const void *in, int outp, int g5, double *red,
 template <typename R>
 int Cphi_eo(double mass, void *out, const void *in, int g5, double *red, const HopTail *tail = nullptr);
 int apply_op(int op, int prec, double mass, void *out, const void *in);
-int apply_op_sqnorm(int op, int prec, double mass, void *out, const void *in, double *red, int *nblocks);
 // one application D (H: gamma_5 D) of an even-odd operator with the |out|^2 (or
 // tail's) partial sums of its last hop in red[0 .. hop_red_blocks(...))
 int apply_eo(bool clover, int prec, double mass, void *out, const void *in, int g5, double *red, const HopTail *tail);
