@@ -4,9 +4,10 @@
 //
 // The recursions are HiRep's.  g5QMR keeps every scalar on the device (alpha,
 // rho, delta, beta and the Givens rotations of every shift live in a state
-// struct; one-block folds update them from the partial sums of the fused
-// vector kernels), so an iteration is the operator plus five kernels and the
-// host reads the state once per chunk of iterations, as the CG does (cg.cu).
+// struct; one-block folds update them from the partial sums of the operator's last
+// hop and of the fused vector kernels), so an iteration is the operator plus four
+// kernels, three iterations are captured as a CUDA graph, and the host reads the
+// state once per graph, one graph behind, as the CG does (cg.cu).
 // MINRES and MRE keep their few scalars on the host.  These solvers are
 // HiRep's choice for the non-hermitian D (force_hmc.c:122-155,
 // calc_prop.c:210-289) and the fallbacks around it.
@@ -82,20 +83,23 @@ struct QLA {
 
 // ---------------------------------------------------------------------------
 // g5QMR_mshift_core (g5QMR_mshift.c:83-279) with the scalars on the device.
-// One iteration (p1, p2, Mp the three rotating directions, q1/q2 per shift):
-//   Mp = M p2 - s_0 p2                      operator + k_q_alpha (<g5 p2, Mp> partials)
-//   alpha = <g5 p2, Mp> / delta              k_q_fold_alpha
-//   Mp -= beta p1 + alpha p2                 k_q_p (|Mp|^2 and <g5 Mp, Mp> partials)
-//   rho, the Givens step of every shift,     k_q_fold_rho (one thread, HiRep's order;
+// The directions are kept as f p with their factor f in the state (p2 = Mp / rho
+// costs no pass over the field); f1, f2 belong to p1, p2 below.  One iteration (p1,
+// p2, Mp the three rotating fields, q1/q2 per shift):
+//   Mp = M p2                                operator; <g5 p2, Mp> partials from its
+//                                            last hop (or k_q_alpha)
+//   alpha = f2^2 <g5 p2, Mp> / delta - s_0    k_q_fold_alpha (<g5 f2 p2, f2 p2> = delta)
+//   Mp = f2 Mp - beta f1 p1 - (alpha + s_0) f2 p2   k_q_p (|Mp|^2 and <g5 Mp, Mp> partials)
+//   rho, the Givens step of every shift,     k_q_fold_rho (HiRep's order;
 //   delta = <g5 Mp, Mp>/rho^2, beta, flags    the convergence and failure tests)
-//   per shift: q_new = d (p1 - t q1 - e q2),  k_q_shift (q_new overwrites q1 in place
-//   out += c2 r q_new; p2 = Mp / rho           and the two q buffers swap roles)
+//   per shift: q_new = d (f1 p1 - t q1 - e q2),  k_q_shift (q_new overwrites q1 in place
+//   out += c2 r q_new                         and the two q buffers swap roles)
 // ---------------------------------------------------------------------------
 constexpr int QMAX = 64;
-constexpr int QMR_CHUNK = 4;  // iterations launched between two reads of the state
+constexpr int QMR_CHUNK = 3;  // iterations per graph (the three directions rotate once) and read of the state
 
 struct QMRState {
-  double alpha, beta, delta, rho, scale, innorm2, err2;
+  double alpha, beta, delta, rho, f1, f2, innorm2, err2;
   int n, iter, max_iter, state, notconv;
   double shift[QMAX], r[QMAX], s1[QMAX], s2[QMAX], c1[QMAX], c2[QMAX];
   double t[QMAX], e[QMAX], d[QMAX], cout[QMAX];  // this iteration's coefficients per shift
@@ -104,7 +108,15 @@ struct QMRState {
 
 __device__ double q_fold(const double *partials, int nblocks, int stride, int off) {
   double v = 0;
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v += partials[(long)b * stride + off];
+  int b = threadIdx.x;
+  for (; b + 3 * (int)blockDim.x < nblocks; b += 4 * blockDim.x) {
+    double u[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) u[k] = partials[(long)(b + k * (int)blockDim.x) * stride + off];
+#pragma unroll
+    for (int k = 0; k < 4; k++) v += u[k];
+  }
+  for (; b < nblocks; b += blockDim.x) v += partials[(long)b * stride + off];
   return block_sum(v);
 }
 
@@ -112,45 +124,44 @@ __device__ __forceinline__ double q_g5(long e, int ld, int nf) {
   return ((int)((e / ld) % (4 * nf)) / nf) < 2 ? 1.0 : -1.0;
 }
 
-// Mp -= s_0 p2 (the shift of the first system, g5QMR_mshift.c:128); partials of
-// <g5 p2, Mp>.  SHIFT false: s_0 = 0 (the host knows the shifts), Mp is only read.
-template <bool SHIFT>
-__global__ void __launch_bounds__(RED_THREADS) k_q_alpha(const QMRState *S, double2 *Mp, const double2 *p2, long n,
+// partials of <g5 p2, Mp>, for the operators whose last hop does not leave them
+__global__ void __launch_bounds__(RED_THREADS) k_q_alpha(const QMRState *S, const double2 *Mp, const double2 *p2, long n,
                                                          int ld, int nf, double *partials) {
   if (S->state != 0) return;
-  const double s0 = S->shift[0];
   double acc = 0.0;
   const long stride = (long)gridDim.x * blockDim.x;
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const double2 a = p2[e];
-    double2 v = Mp[e];
-    if (SHIFT) {
-      rmac(v, -s0, a);
-      Mp[e] = v;
-    }
+    const double2 a = p2[e], v = Mp[e];
     acc += q_g5(e, ld, nf) * (a.x * v.x + a.y * v.y);
   }
   acc = block_sum(acc);
   if (threadIdx.x == 0) partials[blockIdx.x] = acc;
 }
 
+// the first kernel of an iteration to change the state: after the last one it only marks the end
 __global__ void k_q_fold_alpha(QMRState *S, const double *partials, int nblocks) {
-  if (S->state != 0) return;
+  pdl_enter();
+  if (S->state != 0) {
+    if (threadIdx.x == 0 && S->state == 1) S->state = 2;
+    return;
+  }
   const double a = q_fold(partials, nblocks, 1, 0);
-  if (threadIdx.x == 0) S->alpha = a / S->delta;
+  if (threadIdx.x == 0) S->alpha = S->f2 * S->f2 * a / S->delta - S->shift[0];
 }
 
-// Mp -= beta p1 + alpha p2 (g5QMR_mshift.c:131-132); partials of |Mp|^2 and <g5 Mp, Mp>
+// Mp = f2 Mp - beta f1 p1 - (alpha + s_0) f2 p2 (g5QMR_mshift.c:128-132); partials of |Mp|^2 and <g5 Mp, Mp>
 __global__ void __launch_bounds__(RED_THREADS) k_q_p(const QMRState *S, double2 *Mp, const double2 *p1,
                                                      const double2 *p2, long n, int ld, int nf, double *partials) {
+  pdl_enter();
   if (S->state != 0) return;
-  const double beta = S->beta, alpha = S->alpha;
+  const double f2 = S->f2, c1 = -S->beta * S->f1, c2 = -(S->alpha + S->shift[0]) * f2;
   double nrm = 0.0, g5n = 0.0;
   const long stride = (long)gridDim.x * blockDim.x;
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
     double2 v = Mp[e];
-    rmac(v, -beta, p1[e]);
-    rmac(v, -alpha, p2[e]);
+    v = make_double2(f2 * v.x, f2 * v.y);
+    rmac(v, c1, p1[e]);
+    rmac(v, c2, p2[e]);
     Mp[e] = v;
     const double q = v.x * v.x + v.y * v.y;
     nrm += q;
@@ -166,9 +177,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_q_p(const QMRState *S, double2 
 
 // rho, the Givens step of every shift, delta and beta, convergence (g5QMR_mshift.c:135-228)
 __global__ void k_q_fold_rho(QMRState *S, const double *partials, int nblocks) {
+  pdl_enter();
   if (S->state != 0) return;
-  const double nrm = q_fold(partials, nblocks, 2, 0);
-  const double g5n = q_fold(partials, nblocks, 2, 1);
+  const double nrm = q_fold(partials, nblocks, 2, 0), g5n = q_fold(partials, nblocks, 2, 1);
   if (threadIdx.x != 0) return;
   const int iter = ++S->iter;
   const double rho = sqrt(nrm), alpha = S->alpha;
@@ -210,9 +221,10 @@ __global__ void k_q_fold_rho(QMRState *S, const double *partials, int nblocks) {
       --notconv;
     }
   }
-  S->scale = 0.0;
+  S->f1 = S->f2;
+  S->f2 = 1.0;
   if (fabs(rho) > 1.e-13) {
-    S->scale = 1. / rho;
+    S->f2 = 1. / rho;
     const double olddelta = S->delta;
     S->delta = g5n / (rho * rho);
     if (fabs(S->delta) < 1.e-6 || maxm < 1.e-3) notconv = 0;  // the method has failed
@@ -225,13 +237,13 @@ __global__ void k_q_fold_rho(QMRState *S, const double *partials, int nblocks) {
   if (notconv == 0 || (S->max_iter != 0 && iter >= S->max_iter)) S->state = 1;
 }
 
-// per shift: q_new = d (p1 - t q1 - e q2) into q1's buffer, out += c2 r q_new
-// (g5QMR_mshift.c:152-170); then p2 = Mp / rho (:188)
+// per shift: q_new = d (f1 p1 - t q1 - e q2) into q1's buffer, out += c2 r q_new (g5QMR_mshift.c:152-170)
 __global__ void k_q_shift(const QMRState *S, double2 *const *out, double2 *const *qa, double2 *const *qb,
-                          const double2 *p1, double2 *p2, long n) {
+                          const double2 *p1, long n) {
+  pdl_enter();
   if (S->state >= 2) return;
   const int ns = S->n;
-  const double scale = S->scale;
+  const double f1 = S->f1;
   const long stride = (long)gridDim.x * blockDim.x;
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
     const double2 pv = p1[e];
@@ -245,27 +257,24 @@ __global__ void k_q_shift(const QMRState *S, double2 *const *out, double2 *const
       v.x = (-S->t[i] * d) * a.x;
       v.y = (-S->t[i] * d) * a.y;
       rmac(v, -S->e[i] * d, b);
-      rmac(v, d, pv);
+      rmac(v, d * f1, pv);
       q1[e] = v;
       double2 o = out[i][e];
       rmac(o, S->cout[i], v);
       out[i][e] = o;
     }
-    if (scale != 0.0) {
-      double2 v = p2[e];
-      v.x *= scale;
-      v.y *= scale;
-      p2[e] = v;
-    }
   }
 }
 
-__global__ void k_q_advance(QMRState *S) {
-  if (S->state == 1) S->state = 2;
-}
-
 struct QMRWork {
-  QMRState *S = nullptr, *hS = nullptr;
+  QMRState *S = nullptr, *hS = nullptr;  // hS: the states after the last two graphs
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaStream_t cap = nullptr;
+  // the captured iterations and what they were captured for
+  cudaGraphExec_t exec = nullptr;
+  int op = -1, n = 0, v[3] = {-1, -1, -1}, force = -1, pdl = -1, recon = -1;
+  double mass = 0.0;
+  const void *key[9] = {};
   void **d_ptrs = nullptr;  // out[QMAX], qa[QMAX], qb[QMAX]
 };
 static QMRWork QW;
@@ -274,7 +283,110 @@ static void qmr_release_state() {
   if (QW.S) cudaFree(QW.S);
   if (QW.hS) cudaFreeHost(QW.hS);
   if (QW.d_ptrs) cudaFree(QW.d_ptrs);
+  if (QW.exec) cudaGraphExecDestroy(QW.exec);
+  if (QW.cap) cudaStreamDestroy(QW.cap);
+  for (cudaEvent_t ev : QW.ev)
+    if (ev) cudaEventDestroy(ev);
   QW = QMRWork();
+}
+
+// QMR_CHUNK iterations on the fields P (the rotation brings each back to its place)
+static int qmr_iterations(int op, double mass, void *const (&P)[3], long ne, unsigned g) {
+  double2 *const *d_out = (double2 *const *)QW.d_ptrs;
+  double2 *const *d_qa = (double2 *const *)(QW.d_ptrs + QMAX);
+  double2 *const *d_qb = (double2 *const *)(QW.d_ptrs + 2 * QMAX);
+  const bool eo = op == HRGPU_OP_DPHI_EOPRE || op == HRGPU_OP_CPHI_EOPRE, clover = op == HRGPU_OP_CPHI_EOPRE;
+  int ip1 = 0, ip2 = 1, imp = 2;
+  for (int c = 0; c < QMR_CHUNK; c++) {
+    int nb;
+    if (eo && hop_tail_settled(clover, HRGPU_DOUBLE)) {
+      HopTail t;
+      t.red_g5 = 1;
+      QTRY(apply_eo(clover, HRGPU_DOUBLE, mass, P[imp], P[ip2], 0, L.partials, &t));
+      nb = hop_red_blocks(clover, HRGPU_DOUBLE);
+    } else {
+      QTRY(apply_op(op, HRGPU_DOUBLE, mass, P[imp], P[ip2]));
+      k_q_alpha<<<g, RED_THREADS, 0, L.stream>>>(QW.S, (const double2 *)P[imp], (const double2 *)P[ip2], ne, L.ld, L.nf,
+                                                 L.partials);
+      nb = (int)g;
+    }
+    // every kernel after the operator starts while the one before it ends
+    const unsigned th = RED_THREADS;
+    HR_CUDA(launch_after(L.hop_pdl, k_q_fold_alpha, 1u, th, QW.S, L.partials, nb));
+    HR_CUDA(launch_after(L.hop_pdl, k_q_p, g, th, QW.S, (double2 *)P[imp], (const double2 *)P[ip1], (const double2 *)P[ip2],
+                         ne, L.ld, L.nf, L.partials));
+    HR_CUDA(launch_after(L.hop_pdl, k_q_fold_rho, 1u, th, QW.S, L.partials, (int)g));
+    // the three directions rotate: p1 <- p2, p2 <- Mp, Mp <- p1
+    const int o1 = ip1;
+    ip1 = ip2;
+    ip2 = imp;
+    imp = o1;
+    HR_CUDA(launch_after(L.hop_pdl, k_q_shift, g, th, QW.S, d_out, d_qa, d_qb, (const double2 *)P[ip1], ne));
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail_cuda(e, "g5QMR iteration", __FILE__, __LINE__);
+  }
+  return 0;
+}
+
+// The same as a graph, captured once per operator, fields and kernel variants.
+// *mvm: the hops of the chunk, for the caller to count when it is known that they ran.
+static int qmr_chunk(int op, double mass, int n, void *const (&P)[3], long ne, unsigned g, unsigned long *mvm) {
+  const bool clover = op == HRGPU_OP_CPHI_EOPRE || op == HRGPU_OP_CPHI;
+  if (clover) QTRY(clover_prepare(mass, HRGPU_DOUBLE));
+  const int *hv = L.hop_variant[0];
+  const bool settled = L.hop_force >= 0 || (clover ? (hv[EP_CLOV] >= 0 && (op == HRGPU_OP_CPHI || hv[EP_CLOV_INV] >= 0))
+                                                   : hv[EP_AXPY] >= 0);
+  const unsigned long m0 = mvm_count();
+  if (!settled) {  // tunes the hopping kernels
+    const int rc = qmr_iterations(op, mass, P, ne, g);
+    *mvm = mvm_count() - m0;
+    mvm_restore(m0);
+    return rc;
+  }
+  if (op == HRGPU_OP_DPHI_EOPRE || op == HRGPU_OP_CPHI_EOPRE)
+    QTRY(ensure_tmp(&L.tmp_o, spinor_bytes(HRGPU_EVEN, HRGPU_DOUBLE)));
+  const void *key[9] = {P[0], P[1], P[2], QW.S, QW.d_ptrs, L.U, L.tmp_o, L.partials, L.cl_idg};
+  const int recon = L.recon_allow ? L.recon12 : 0;
+  bool same = QW.exec && QW.op == op && QW.n == n && QW.mass == mass && QW.force == L.hop_force && QW.pdl == (int)L.hop_pdl &&
+              QW.recon == recon;
+  for (int i = 0; i < 3 && same; i++) same = QW.v[i] == hv[i];
+  for (int i = 0; i < 9 && same; i++) same = QW.key[i] == key[i];
+  const unsigned long per = QMR_CHUNK * 2ul;  // two hops per application of D, even-odd or full
+  if (!same) {
+    if (QW.exec) cudaGraphExecDestroy(QW.exec);
+    QW.exec = nullptr;
+    if (!QW.cap) HR_CUDA(cudaStreamCreateWithFlags(&QW.cap, cudaStreamNonBlocking));
+    cudaStream_t saved = L.stream;
+    cudaGraph_t graph = nullptr;
+    HR_CUDA(cudaStreamBeginCapture(QW.cap, cudaStreamCaptureModeRelaxed));
+    L.stream = QW.cap;
+    const int rc = qmr_iterations(op, mass, P, ne, g);
+    L.stream = saved;
+    cudaError_t e = cudaStreamEndCapture(QW.cap, &graph);
+    mvm_restore(m0);  // nothing ran yet
+    if (rc) {
+      if (graph) cudaGraphDestroy(graph);
+      return rc;
+    }
+    if (e != cudaSuccess) return fail_cuda(e, "g5QMR capture", __FILE__, __LINE__);
+    e = cudaGraphInstantiate(&QW.exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (e != cudaSuccess) {
+      QW.exec = nullptr;
+      return fail_cuda(e, "g5QMR graph instantiate", __FILE__, __LINE__);
+    }
+    QW.op = op;
+    QW.n = n;
+    QW.mass = mass;
+    QW.force = L.hop_force;
+    QW.pdl = (int)L.hop_pdl;
+    QW.recon = recon;
+    for (int i = 0; i < 3; i++) QW.v[i] = hv[i];
+    for (int i = 0; i < 9; i++) QW.key[i] = key[i];
+  }
+  HR_CUDA(cudaGraphLaunch(QW.exec, L.stream));
+  *mvm = per;
+  return 0;
 }
 
 // valid[i]: the true residual of shift i is below err2.  Returns the MVM count in *iters.
@@ -286,11 +398,12 @@ static int g5qmr_core(short *valid, int op, double mass, int n, const double *sh
   QTRY(qpool(2 * n + 3, spinor_bytes(par, HRGPU_DOUBLE)));
   if (!QW.S) {
     HR_CUDA(cudaMalloc(&QW.S, sizeof(QMRState)));
-    HR_CUDA(cudaMallocHost(&QW.hS, sizeof(QMRState)));
+    HR_CUDA(cudaMallocHost(&QW.hS, 2 * sizeof(QMRState)));
+    for (cudaEvent_t &ev : QW.ev) HR_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     HR_CUDA(cudaMalloc(&QW.d_ptrs, sizeof(void *) * 3 * QMAX));
   }
   void *P[3] = {QP.f[2 * n], QP.f[2 * n + 1], QP.f[2 * n + 2]};  // p1, p2, Mp
-  int ip1 = 0, ip2 = 1, imp = 2;
+  const int ip1 = 0, ip2 = 1, imp = 2;
   int cgiter = 0;
   double innorm2, rho, delta;
   QTRY(la.op(LA_COPY, P[ip2], in));
@@ -312,24 +425,26 @@ static int g5qmr_core(short *valid, int op, double mass, int n, const double *sh
   QTRY(la.g5re(P[ip2], P[ip2], &delta));
   HR_REQUIRE(fabs(delta) >= 1.e-28, HRGPU_E_ARG,
              "g5QMR: gamma_5 norm of the initial guess is zero, change the initial guess");
-  QMRState &h = *QW.hS;
-  memset(&h, 0, sizeof(QMRState));
-  h.alpha = 0;
-  h.beta = delta;
-  h.delta = delta;
-  h.innorm2 = innorm2;
-  h.err2 = err2;
-  h.n = n;
-  h.max_iter = max_iter;
-  h.notconv = n;
+  // (the reductions above have waited for the stream, so no copy into hS is in flight)
+  QMRState &h0 = QW.hS[0];
+  memset(&h0, 0, sizeof(QMRState));
+  h0.alpha = 0;
+  h0.beta = delta;
+  h0.f1 = h0.f2 = 1.0;
+  h0.delta = delta;
+  h0.innorm2 = innorm2;
+  h0.err2 = err2;
+  h0.n = n;
+  h0.max_iter = max_iter;
+  h0.notconv = n;
   for (int i = 0; i < n; i++) {
-    h.shift[i] = shift[i];
-    h.r[i] = rho;
-    h.c1[i] = h.c2[i] = 1.;
-    h.s1[i] = h.s2[i] = 0.;
-    h.flag[i] = 1;
+    h0.shift[i] = shift[i];
+    h0.r[i] = rho;
+    h0.c1[i] = h0.c2[i] = 1.;
+    h0.s1[i] = h0.s2[i] = 0.;
+    h0.flag[i] = 1;
   }
-  HR_CUDA(cudaMemcpyAsync(QW.S, &h, sizeof(QMRState), cudaMemcpyHostToDevice, L.stream));
+  HR_CUDA(cudaMemcpyAsync(QW.S, &h0, sizeof(QMRState), cudaMemcpyHostToDevice, L.stream));
   void *ptrs[3 * QMAX];
   for (int i = 0; i < n; i++) {
     ptrs[i] = out[i];
@@ -337,57 +452,38 @@ static int g5qmr_core(short *valid, int op, double mass, int n, const double *sh
     ptrs[2 * QMAX + i] = QP.f[n + i];
   }
   HR_CUDA(cudaMemcpyAsync(QW.d_ptrs, ptrs, sizeof(void *) * 3 * QMAX, cudaMemcpyHostToDevice, L.stream));
-  double2 *const *d_out = (double2 *const *)QW.d_ptrs;
-  double2 *const *d_qa = (double2 *const *)(QW.d_ptrs + QMAX);
-  double2 *const *d_qb = (double2 *const *)(QW.d_ptrs + 2 * QMAX);
   const long ne = (long)spinor_elems(par);
   long gb = (ne + RED_THREADS - 1) / RED_THREADS;
   const unsigned g = (unsigned)(gb < RED_MAX_BLOCKS ? gb : RED_MAX_BLOCKS);
+  // one graph is in flight behind the one whose state is read; its kernels return
+  // at once after the last iteration
   const unsigned long m0 = mvm_count();
-  unsigned long per_it = 0;
-  int rc = 0;
+  unsigned long mvm = 0;
   L.cur_stop = &QW.S->state;
-  for (;;) {
-    for (int c = 0; c < QMR_CHUNK && !rc; c++) {
-      const unsigned long mb = mvm_count();
-      rc = apply_op(op, HRGPU_DOUBLE, mass, P[imp], P[ip2]);
-      if (rc) break;
-      per_it = mvm_count() - mb;
-      if (shift[0] != 0.0)
-        k_q_alpha<true><<<g, RED_THREADS, 0, L.stream>>>(QW.S, (double2 *)P[imp], (const double2 *)P[ip2], ne, L.ld,
-                                                         L.nf, L.partials);
-      else
-        k_q_alpha<false><<<g, RED_THREADS, 0, L.stream>>>(QW.S, (double2 *)P[imp], (const double2 *)P[ip2], ne, L.ld,
-                                                          L.nf, L.partials);
-      k_q_fold_alpha<<<1, RED_THREADS, 0, L.stream>>>(QW.S, L.partials, g);
-      k_q_p<<<g, RED_THREADS, 0, L.stream>>>(QW.S, (double2 *)P[imp], (const double2 *)P[ip1],
-                                             (const double2 *)P[ip2], ne, L.ld, L.nf, L.partials);
-      k_q_fold_rho<<<1, RED_THREADS, 0, L.stream>>>(QW.S, L.partials, g);
-      // the three directions rotate: p1 <- p2, p2 <- Mp, Mp <- p1
-      const int o1 = ip1;
-      ip1 = ip2;
-      ip2 = imp;
-      imp = o1;
-      k_q_shift<<<g, RED_THREADS, 0, L.stream>>>(QW.S, d_out, d_qa, d_qb, (const double2 *)P[ip1], (double2 *)P[ip2],
-                                                 ne);
-      k_q_advance<<<1, 1, 0, L.stream>>>(QW.S);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) rc = fail_cuda(e, "g5QMR iteration", __FILE__, __LINE__);
-    }
+  auto launch = [&](int b) -> int {
+    if (int q = qmr_chunk(op, mass, n, P, ne, g, &mvm)) return q;
+    HR_CUDA(cudaMemcpyAsync(&QW.hS[b], QW.S, sizeof(QMRState), cudaMemcpyDeviceToHost, L.stream));
+    HR_CUDA(cudaEventRecord(QW.ev[b], L.stream));
+    return 0;
+  };
+  int rc = launch(0), cur = 0;
+  while (!rc) {
+    rc = launch(cur ^ 1);
     if (rc) break;
-    cudaError_t e = cudaMemcpyAsync(&h, QW.S, sizeof(QMRState), cudaMemcpyDeviceToHost, L.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(L.stream);
+    cudaError_t e = cudaEventSynchronize(QW.ev[cur]);
     if (e != cudaSuccess) {
       rc = fail_cuda(e, "g5QMR state readback", __FILE__, __LINE__);
       break;
     }
-    if (h.state != 0) break;
+    if (QW.hS[cur].state != 0) break;
+    cur ^= 1;
   }
   L.cur_stop = nullptr;
   if (rc) return rc;
-  mvm_restore(m0 + (unsigned long)h.iter * per_it);  // the launches after convergence did nothing
+  const QMRState &h = QW.hS[cur];
+  mvm_restore(m0 + (unsigned long)h.iter * (mvm / QMR_CHUNK));  // the launches after convergence did nothing
   cgiter = h.iter;
-  void *Mp = P[imp];
+  void *Mp = P[2];
   for (int i = 0; i < n; i++) {
     QTRY(apply_op(op, HRGPU_DOUBLE, mass, Mp, out[i]));
     ++cgiter;
