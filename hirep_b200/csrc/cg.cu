@@ -8,13 +8,16 @@
 //   H k (two hops, the last with the |H k|^2 = <k, H^2 k> partials) ->
 //   fold_alpha, beside the first hop of the second H -> its last hop, which adds
 //   omega H^2 k to r instead of writing it and leaves the |r|^2 partials ->
-//   fold_lambda -> update (k = gamma k + r, x_i += c_i p_i, p_i = d_i p_i + z3_i r)
+//   fold_lambda -> k = gamma k + r
+// and the shifted systems (x_i += c_i p_i, p_i = d_i p_i + z3_i r), which only follow
+// the recursion, are brought up to date once per CG_CHUNK iterations.
 // With another operator the products and r += omega M k are kernels of their own.
 // The host launches several iterations at a time (a captured CUDA graph), one chunk
 // ahead of the state that it reads.  When fold_lambda finds the stopping condition it marks the
 // state; the remaining kernels of that iteration finish it exactly as HiRep's
 // loop body would, and every kernel of later iterations returns at once, so the
 // solution and the iteration count are those of HiRep's loop.
+#include <cstddef>
 #include <type_traits>
 #include <vector>
 
@@ -30,8 +33,13 @@ constexpr int CG_HARD_LIMIT = 200000;  // iterations, when the caller sets no ma
 struct CGState {
   double omega, oldomega, gamma, alpha, lambda, delta, innorm2, err2;
   int n, state, iter, max_iter, notconv, flt;
-  double shift[MAXS], z1[MAXS], z2[MAXS], z3[MAXS], cx[MAXS], cp[MAXS];
+  double shift[MAXS], z1[MAXS], z2[MAXS], z3[MAXS];
   int flag[MAXS];
+  // the last iterations' coefficients of the shifted systems, not yet applied to the fields:
+  // x_i += cx p_i, then p_i = cp p_i + pz r where pf is set
+  int pend;  // how many
+  double cx[CG_CHUNK][MAXS], cp[CG_CHUNK][MAXS], pz[CG_CHUNK][MAXS];
+  int pf[CG_CHUNK][MAXS];
 };
 
 constexpr int FOLD_THREADS = 512;
@@ -54,7 +62,10 @@ __device__ double fold_partials(const double *partials, int nblocks, int stride)
 // alpha = <k, Mk>; omega = -delta/alpha; z3 and the solution coefficients
 // (cg_mshift.c:82-91), one thread per shift.  The first kernel of an iteration to
 // change the state: an iteration after the one that converged only marks the end.
-__global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_alpha(CGState *S, const double *partials, int nblocks, int stride) {
+// slot: the iteration's place among those kept for the shifted systems.
+__global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_alpha(CGState *S, const double *partials, int nblocks, int stride,
+                                                                int slot) {
+  if (slot == 0 && threadIdx.x == 0) S->pend = 0;
   if (S->state != 0) {
     if (threadIdx.x == 0 && S->state == 1) S->state = 2;
     return;
@@ -68,9 +79,9 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_alpha(CGState *S, cons
       const double z1 = S->z1[i], z2 = S->z2[i];
       const double z3 = oldomega * z1 * z2 / (omega * gamma * (z1 - z2) + z1 * oldomega * (1. + S->shift[i] * omega));
       S->z3[i] = z3;
-      S->cx[i] = -omega * z3 / z2;
+      S->cx[slot][i] = -omega * z3 / z2;
     } else {
-      S->cx[i] = 0.0;
+      S->cx[slot][i] = 0.0;
     }
   }
   __syncthreads();
@@ -86,7 +97,7 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_alpha(CGState *S, cons
 }
 
 // lambda = |r|^2, gamma, convergence flags (cg_mshift.c:92-111; cg_mshift_flt.c:96-118)
-__global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_lambda(CGState *S, const double *partials, int nblocks) {
+__global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_lambda(CGState *S, const double *partials, int nblocks, int slot) {
   pdl_enter();
   if (S->state != 0) return;
   const double lambda = fold_partials(partials, nblocks, 1);
@@ -103,9 +114,11 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_lambda(CGState *S, con
       open = flag;
     }
     // a shift that converged in this iteration keeps its z's, and gets its last x in the update
+    S->pf[slot][i] = flag;
     if (flag) {
       const double z2 = S->z2[i];
-      S->cp[i] = gamma * z3 * z3 / (z2 * z2);
+      S->cp[slot][i] = gamma * z3 * z3 / (z2 * z2);
+      S->pz[slot][i] = z3;
       S->z1[i] = z2;
       S->z2[i] = z3;
     }
@@ -117,14 +130,16 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_lambda(CGState *S, con
     S->delta = lambda;
     S->notconv = notconv;
     S->iter++;
+    if (isfinite(lambda)) S->pend = slot + 1;
     if (!isfinite(lambda)) S->state = 3;
     else if (notconv == 0 || (S->max_iter != 0 && S->iter >= S->max_iter)) S->state = 1;
   }
 }
 
-// r += omega Mk with |r|^2 partials, for the operators whose last hop does not do it
+// rn = r + omega Mk (rn may be r) with |rn|^2 partials, for the operators whose last hop does not do it
 template <typename V>
-__global__ void __launch_bounds__(RED_THREADS) k_cg_update_r(CGState *S, V *r, const V *Mk, long n, double *partials) {
+__global__ void __launch_bounds__(RED_THREADS) k_cg_update_r(CGState *S, V *rn, const V *r, const V *Mk, long n,
+                                                             double *partials) {
   if (S->state != 0) return;
   const double omega = S->omega;
   double nrm = 0.0;
@@ -132,7 +147,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_update_r(CGState *S, V *r, c
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
     V rv = r[e];
     rmac(rv, (decltype(rv.x))omega, Mk[e]);
-    r[e] = rv;
+    rn[e] = rv;
     nrm += (double)rv.x * rv.x + (double)rv.y * rv.y;
   }
   nrm = block_sum(nrm);
@@ -147,45 +162,76 @@ __device__ __forceinline__ float4 fma_r(float a, float4 x, float4 y) {
 __device__ __forceinline__ double2 mul_r(double a, double2 x) { return make_double2(a * x.x, a * x.y); }
 __device__ __forceinline__ float4 mul_r(float a, float4 x) { return make_float4(a * x.x, a * x.y, a * x.z, a * x.w); }
 
-// x_i += cx_i p_i and p_i = cp_i p_i + z3_i r for every shift, k = gamma k + r: p_i
-// is read once for both.  one: a single unshifted system, whose p_i is k (every z
-// is 1), so that k serves for both and p_0 is not touched.
+// k = gamma k + r.  one: a single unshifted system, whose p_0 is k (every z is 1): x_0 += cx_0 k
+// as well, and p_0 is not touched.
 // W: 16-byte words.  (FP32 solves run on the library's own fields only; an FP64
 // complex number is one word, so a caller's field needs no more than its own alignment.)
 template <typename W, typename R, bool PDL>
-__global__ void __launch_bounds__(RED_THREADS) k_cg_update(const CGState *S, W *const *x, W *const *p, W *k, const W *r, long n,
-                                                           int one) {
+__global__ void __launch_bounds__(RED_THREADS) k_cg_update(const CGState *S, W *const *x, W *k, const W *r, long n, int one) {
   if (PDL) pdl_enter();
   if (S->state >= 2) return;
-  __shared__ R cx[MAXS], cp[MAXS], z3[MAXS];
-  __shared__ int flag[MAXS];
+  const R gamma = (R)S->gamma, cx = (R)S->cx[0][0];
+  W *x0 = x[0];
+  const long stride = (long)gridDim.x * blockDim.x;
+  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const W rv = r[e], kv = k[e];
+    if (one) x0[e] = fma_r(cx, kv, x0[e]);
+    k[e] = fma_r(gamma, kv, rv);
+  }
+}
+
+template <typename W>
+struct CGRing {
+  const W *r[CG_CHUNK];
+};
+
+// The iterations kept in S (pend of them, their residuals in ring) applied to every shifted
+// system: x_i += cx p_i, p_i = cp p_i + pz r, one after the other in registers, so the
+// results are bit for bit those of an update in each iteration.  Such an update is bound by HBM:
+// 4n + 3 vectors per iteration (76 us, 6.6 TB/s, for 10 shifts on 16^4 with NF=6 in FP64);
+// this is 4n + CG_CHUNK per CG_CHUNK iterations, with k alone in between.
+template <typename W, typename R>
+__global__ void __launch_bounds__(RED_THREADS) k_cg_shifts(const CGState *S, W *const *x, W *const *p, CGRing<W> ring, long n) {
+  const int pend = S->pend;
+  if (pend == 0) return;
+  __shared__ R cx[CG_CHUNK][MAXS], cp[CG_CHUNK][MAXS], pz[CG_CHUNK][MAXS];
+  __shared__ int pf[CG_CHUNK][MAXS], act[MAXS];  // act: 0 converged before, 1 x only, 2 x and p
   __shared__ W *px[MAXS], *pp[MAXS];
   const int ns = S->n;
-  const R gamma = (R)S->gamma;
   for (int i = threadIdx.x; i < ns; i += blockDim.x) {
-    cx[i] = (R)S->cx[i];
-    cp[i] = (R)S->cp[i];
-    z3[i] = (R)S->z3[i];
-    flag[i] = S->flag[i];
+    int a = 0;
+    for (int c = 0; c < CG_CHUNK; c++) {
+      const bool in = c < pend;
+      cx[c][i] = in ? (R)S->cx[c][i] : (R)0;
+      pf[c][i] = in && cx[c][i] != (R)0 ? S->pf[c][i] : 0;
+      cp[c][i] = pf[c][i] ? (R)S->cp[c][i] : (R)0;
+      pz[c][i] = pf[c][i] ? (R)S->pz[c][i] : (R)0;
+      if (pf[c][i]) a = 2;
+      else if (cx[c][i] != (R)0 && a == 0) a = 1;
+    }
+    act[i] = a;
     px[i] = x[i];
     pp[i] = p[i];
   }
   __syncthreads();
   const long stride = (long)gridDim.x * blockDim.x;
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const W rv = r[e], kv = k[e];
-    if (one) {
-      px[0][e] = fma_r(cx[0], kv, px[0][e]);
-    } else {
+    W rv[CG_CHUNK];
+#pragma unroll
+    for (int c = 0; c < CG_CHUNK; c++) rv[c] = ring.r[c < pend ? c : 0][e];
 #pragma unroll 2
-      for (int i = 0; i < ns; i++) {
-        if (cx[i] == (R)0) continue;
-        const W pv = pp[i][e];
-        px[i][e] = fma_r(cx[i], pv, px[i][e]);
-        if (flag[i]) pp[i][e] = fma_r(z3[i], rv, mul_r(cp[i], pv));
+    for (int i = 0; i < ns; i++) {
+      if (act[i] == 0) continue;
+      W pv = pp[i][e], xv = px[i][e];
+#pragma unroll
+      for (int c = 0; c < CG_CHUNK; c++) {
+        if (cx[c][i] == (R)0) continue;
+        xv = fma_r(cx[c][i], pv, xv);
+        if (pf[c][i]) pv = fma_r(pz[c][i], rv[c], mul_r(cp[c][i], pv));
       }
+      px[i][e] = xv;
+      if (act[i] == 2) pp[i][e] = pv;
     }
-    k[e] = fma_r(gamma, kv, rv);
   }
 }
 
@@ -210,7 +256,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_dot(const CGState *S, const 
 // workspace (cached between calls, grown on demand)
 // ---------------------------------------------------------------------------
 struct CGWork {
-  std::vector<void *> bufs;  // p[0..n-1], k, r, Mk
+  std::vector<void *> bufs;  // p[0..n-1], k, r, Mk, and where memory allows CG_CHUNK - 1 more residuals
   size_t bytes = 0;
   CGState *S = nullptr;
   CGState *hS = nullptr;  // pinned host copies of the last two chunks' states
@@ -248,8 +294,24 @@ static int cg_workspace(int prec, int nvec, size_t bytes) {
   return 0;
 }
 
+// CG_CHUNK - 1 more residuals behind the first nvec fields, where they leave as much again
+// free: true if they are there.  Without them the solve runs as well, updating every iteration.
+static bool cg_more_residuals(CGWork &w, int nvec) {
+  while ((int)w.bufs.size() < nvec + CG_CHUNK - 1) {
+    size_t avail = 0, total = 0;
+    void *b = nullptr;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail / 2 < (CG_CHUNK - 1) * w.bytes ||
+        cudaMalloc(&b, w.bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    w.bufs.push_back(b);
+  }
+  return true;
+}
+
 // The chunk of iterations as a CUDA graph, captured once per (operator, mass,
-// work buffers, kernel variants, link storage) and replayed: ten launches per
+// work buffers, kernel variants, link storage) and replayed: eight launches per
 // iteration, most of them small, cost more in launch gaps than in work.  The
 // graph reads the links and clover blocks at replay; the clover blocks (for
 // this mass) and the BF16 link copy are brought up to date before each replay.
@@ -259,8 +321,8 @@ static int cg_workspace(int prec, int nvec, size_t bytes) {
 struct CGGraph {
   int op = -1;
   double mass = 0;
-  const void *ptrs[10] = {};
-  int v[3] = {-1, -1, -1}, force = -1, flt_links = -1, pdl = -1, recon = -1, one = -1;
+  const void *ptrs[9 + CG_CHUNK] = {};
+  int v[3] = {-1, -1, -1}, force = -1, flt_links = -1, pdl = -1, recon = -1, one = -1, keep = -1;
   unsigned long mvm = 0;  // hop launches in one replay (the MVM counter)
   cudaGraphExec_t exec = nullptr;
 };
@@ -312,10 +374,11 @@ static unsigned red_grid(long n) {
 }
 
 // CG_CHUNK iterations, launched one kernel at a time.  side: a second stream of the
-// capture in progress for the fold beside a hop, or nullptr.
+// capture in progress for the fold beside a hop, or nullptr.  r: the residual after iteration
+// c is r[c % keep]; the shifted systems are updated when keep of them are there.
 template <typename R>
-static int cg_iterations(int op, int prec, double mass, CGWork &w, void *k, void *r, void *Mk, long ne, unsigned g,
-                         int one, cudaStream_t side) {
+static int cg_iterations(int op, int prec, double mass, CGWork &w, void *k, void *const *r, int keep, void *Mk, long ne,
+                         unsigned g, int one, cudaStream_t side) {
   typedef typename C2<R>::T V;
   typedef typename std::conditional<sizeof(R) == 8, double2, float4>::type W;
   const long nw = ne * (long)sizeof(V) / (long)sizeof(W);
@@ -325,8 +388,13 @@ static int cg_iterations(int op, int prec, double mass, CGWork &w, void *k, void
   const bool clover = op == HRGPU_OP_G5CPHI_EOPRE_SQ;
   const bool small = eo && L.hop_pdl && hop_small(clover, prec);
   double *part2 = L.partials + L.npart / 2;  // |r|^2, while the |Hk|^2 ones may still be read
+  CGRing<W> ring;
+  for (int c = 0; c < CG_CHUNK; c++) ring.r[c] = (const W *)r[c % keep];
   for (int c = 0; c < CG_CHUNK; c++) {
     unsigned nlam = g;
+    const int slot = c % keep;
+    const void *r0 = r[(slot + keep - 1) % keep];
+    void *r1 = r[slot];
     if (eo) {
       // alpha = <k, H^2 k> = |H k|^2 from the first H's partials
       void *tmp = eo_tmp(prec);
@@ -339,32 +407,35 @@ static int cg_iterations(int op, int prec, double mass, CGWork &w, void *k, void
         HR_CUDA(cudaEventRecord(cg_ev[0], L.stream));
         HR_CUDA(cudaStreamWaitEvent(fs, cg_ev[0], 0));
       }
-      k_cg_fold_alpha<<<1, FOLD_THREADS, 0, fs>>>(w.S, L.partials, nb, 1);
+      k_cg_fold_alpha<<<1, FOLD_THREADS, 0, fs>>>(w.S, L.partials, nb, 1, slot);
       if (fs != L.stream) HR_CUDA(cudaEventRecord(cg_ev[1], fs));
       if (tail) {
         HopTail t;
-        t.racc = r;
+        t.racc = r0;
         t.omega = &w.S->omega;
         t.no_pdl = fs != L.stream;
         // the second H, joined by the fold before its last hop
         if (int q = eo_stage<R>(clover, mass, 0, HRGPU_EVEN, Mk, tmp, 1, nullptr, 0, -1)) return q;
         if (fs != L.stream) HR_CUDA(cudaStreamWaitEvent(L.stream, cg_ev[1], 0));
-        if (int q = eo_stage<R>(clover, mass, 1, HRGPU_EVEN, Mk, tmp, 1, part2, 0, -1, &t)) return q;
+        if (int q = eo_stage<R>(clover, mass, 1, HRGPU_EVEN, r1, tmp, 1, part2, 0, -1, &t)) return q;
         nlam = (unsigned)nb;
       } else {
         if (int q = apply_eo(clover, prec, mass, Mk, tmp, 1, nullptr, nullptr)) return q;
-        k_cg_update_r<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (V *)r, (const V *)Mk, ne, part2);
+        k_cg_update_r<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (V *)r1, (const V *)r0, (const V *)Mk, ne, part2);
       }
     } else {
       if (int q = apply_op(op, prec, mass, Mk, k)) return q;
       k_cg_dot<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (const V *)k, (const V *)Mk, ne, L.partials);
-      k_cg_fold_alpha<<<1, FOLD_THREADS, 0, L.stream>>>(w.S, L.partials, g, 2);
-      k_cg_update_r<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (V *)r, (const V *)Mk, ne, part2);
+      k_cg_fold_alpha<<<1, FOLD_THREADS, 0, L.stream>>>(w.S, L.partials, g, 2, slot);
+      k_cg_update_r<V><<<g, RED_THREADS, 0, L.stream>>>(w.S, (V *)r1, (const V *)r0, (const V *)Mk, ne, part2);
     }
     // on a small lattice, where the launches count, these start while the kernel before ends
     const bool pdl = side && small;
-    HR_CUDA(launch_after(pdl, k_cg_fold_lambda, 1u, (unsigned)FOLD_THREADS, w.S, part2, (int)nlam));
-    HR_CUDA(launch_after(pdl, pdl ? k_cg_update<W, R, true> : k_cg_update<W, R, false>, red_grid(nw), (unsigned)RED_THREADS, w.S, dx, dp, (W *)k, (const W *)r, nw, one));
+    HR_CUDA(launch_after(pdl, k_cg_fold_lambda, 1u, (unsigned)FOLD_THREADS, w.S, part2, (int)nlam, slot));
+    HR_CUDA(launch_after(pdl, pdl ? k_cg_update<W, R, true> : k_cg_update<W, R, false>, red_grid(nw), (unsigned)RED_THREADS,
+                         w.S, dx, (W *)k, (const W *)r1, nw, one));
+    if (!one && slot == keep - 1)
+      k_cg_shifts<W, R><<<red_grid(nw), RED_THREADS, 0, L.stream>>>(w.S, dx, dp, ring, nw);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "cg iteration", __FILE__, __LINE__);
   }
@@ -376,8 +447,8 @@ static bool op_is_clover(int op) {
 }
 // *mvm: the hops of the chunk launched, for the caller to count when it is known that they ran
 template <typename R>
-static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, void *Mk, long ne, unsigned g, int one,
-                    unsigned long *mvm) {
+static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *const *r, int keep, void *Mk, long ne,
+                    unsigned g, int one, unsigned long *mvm) {
   if (op_is_clover(op))
     if (int rc = clover_prepare(mass, prec)) return rc;
   if (prec == HRGPU_FLOAT && L.flt_links == HRGPU_LINKS_BF16)
@@ -390,21 +461,22 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, 
                                                    : L.hop_variant[pi][EP_AXPY] >= 0);
   if (!settled) {  // tunes the hopping kernels
     const unsigned long m0 = mvm_count();
-    const int rc = cg_iterations<R>(op, prec, mass, w, k, r, Mk, ne, g, one, nullptr);
+    const int rc = cg_iterations<R>(op, prec, mass, w, k, r, keep, Mk, ne, g, one, nullptr);
     *mvm = mvm_count() - m0;
     mvm_restore(m0);
     return rc;
   }
   const void *links = prec == HRGPU_DOUBLE ? (const void *)L.U
                                            : (L.flt_links == HRGPU_LINKS_BF16 ? (const void *)L.Ubf : (const void *)L.Uf);
-  const void *ptrs[10] = {k, r, Mk, w.S, w.d_ptrs, L.partials, links, L.cur_stop,
+  const void *ptrs[9 + CG_CHUNK] = {k, Mk, w.S, w.d_ptrs, L.partials, links, L.cur_stop,
                           prec == HRGPU_DOUBLE ? L.tmp_e : L.tmp_e_f, prec == HRGPU_DOUBLE ? L.tmp_o : L.tmp_o_f};
+  for (int c = 0; c < CG_CHUNK; c++) ptrs[9 + c] = r[c % keep];
   CGGraph &c = CGG[prec];
   const int recon = L.recon_allow ? L.recon12 : 0;
   bool same = c.exec && c.op == op && c.mass == mass && c.force == L.hop_force && c.flt_links == L.flt_links &&
-              c.pdl == (int)L.hop_pdl && c.recon == recon && c.one == one;
+              c.pdl == (int)L.hop_pdl && c.recon == recon && c.one == one && c.keep == keep;
   for (int i = 0; i < 3 && same; i++) same = c.v[i] == L.hop_variant[pi][i];
-  for (int i = 0; i < 10 && same; i++) same = c.ptrs[i] == ptrs[i];
+  for (int i = 0; i < 9 + CG_CHUNK && same; i++) same = c.ptrs[i] == ptrs[i];
   if (!same) {
     drop_cg_graph(c);
     if (!cg_cap) {
@@ -417,7 +489,7 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, 
     cudaStream_t saved = L.stream;
     HR_CUDA(cudaStreamBeginCapture(cg_cap, cudaStreamCaptureModeRelaxed));
     L.stream = cg_cap;
-    int rc = cg_iterations<R>(op, prec, mass, w, k, r, Mk, ne, g, one, cg_cap2);
+    int rc = cg_iterations<R>(op, prec, mass, w, k, r, keep, Mk, ne, g, one, cg_cap2);
     L.stream = saved;
     cudaError_t e = cudaStreamEndCapture(cg_cap, &graph);
     const unsigned long dm = mvm_count() - m0;
@@ -440,8 +512,9 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *r, 
     c.pdl = (int)L.hop_pdl;
     c.recon = recon;
     c.one = one;
+    c.keep = keep;
     for (int i = 0; i < 3; i++) c.v[i] = L.hop_variant[pi][i];
-    for (int i = 0; i < 10; i++) c.ptrs[i] = ptrs[i];
+    for (int i = 0; i < 9 + CG_CHUNK; i++) c.ptrs[i] = ptrs[i];
     c.mvm = dm;
   }
   HR_CUDA(cudaGraphLaunch(c.exec, L.stream));
@@ -519,15 +592,20 @@ static int cg_core(int op, double mass, int n, const double *shift, double err2,
   }
   HR_CUDA(cudaMemcpyAsync(w.d_ptrs, ptrs, sizeof(void *) * 2 * MAXS, cudaMemcpyHostToDevice, L.stream));
   const unsigned g = red_grid(ne);
+  const int one = n == 1 && shift[0] == 0.0;
+  // residuals of the last CG_CHUNK iterations where the shifted systems can wait for them
+  void *ring[CG_CHUNK] = {r, r, r, r};
+  const int keep = !one && cg_more_residuals(w, n + 3) ? CG_CHUNK : 1;
+  if (keep > 1)
+    for (int c = 0; c < CG_CHUNK - 1; c++) ring[c] = w.bufs[n + 3 + c];  // the first is in ring[CG_CHUNK - 1] = r
   L.cur_stop = &w.S->state;
   int rc = 0;
   // one chunk is in flight behind the one whose state is read; the kernels of a
   // chunk that follows the last iteration return at once and its hops are not counted
-  const int one = n == 1 && shift[0] == 0.0;
   unsigned long mvm[2] = {0, 0};
   auto launch = [&](int b) -> int {
-    if (int q = cg_chunk<R>(op, prec, mass, w, k, r, Mk, ne, g, one, &mvm[b])) return q;
-    HR_CUDA(cudaMemcpyAsync(&w.hS[b], w.S, sizeof(CGState), cudaMemcpyDeviceToHost, L.stream));
+    if (int q = cg_chunk<R>(op, prec, mass, w, k, ring, keep, Mk, ne, g, one, &mvm[b])) return q;
+    HR_CUDA(cudaMemcpyAsync(&w.hS[b], w.S, offsetof(CGState, cx), cudaMemcpyDeviceToHost, L.stream));
     HR_CUDA(cudaEventRecord(w.ev[b], L.stream));
     return 0;
   };

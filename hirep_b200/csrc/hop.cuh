@@ -47,7 +47,7 @@ struct HopArgs {
   int pre;           // the launch before this one is a hop of the same operator: what no hop writes
                      // (links, clover blocks, aux) may be read before waiting for it (k_hop_dir)
   // second hop of an operator inside an inverter (hop_tail_ok's variants):
-  void *racc;           // non-null: racc += *omega * result instead of out = result, red is of the new racc
+  const void *racc;     // non-null: out = racc + *omega * result (racc may be out), red is of that
   const double *omega;
   int no_pdl;           // a launch that joins two branches of a graph
   int red_g5;           // red is Re <gamma_5 aux, result> instead of |result|^2
@@ -56,7 +56,7 @@ struct HopArgs {
 
 // the inverters' forms of an operator's last hop (see HopArgs)
 struct HopTail {
-  void *racc = nullptr;
+  const void *racc = nullptr;
   const double *omega = nullptr;
   int red_g5 = 0, no_pdl = 0, pre = 0;
 };
@@ -646,11 +646,11 @@ __device__ __forceinline__ double hop_site(const HopArgs<R> &a, const int cb, co
     const R sg = a.g5 ? (R)-1 : (R)1;
     if (TAIL && a.racc) {
       const R om = (R)*a.omega;
-      V *rp = (V *)a.racc + cb;
+      const V *rp = (const V *)a.racc + cb;
       auto acc = [&](int c, V v) {
         V r = rp[(long)c * ld];
         rmac(r, om, v);
-        rp[(long)c * ld] = r;
+        out[(long)c * ld] = r;
         nrm += (double)r.x * r.x + (double)r.y * r.y;
       };
 #pragma unroll

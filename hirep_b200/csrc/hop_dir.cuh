@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(HD_THREADS, MINB) k_hop_dir(HopArgs<R> a) {
         acc[k] = EP == EP_CLOV ? cadd(acc[k], y) : y;
       }
     }
-    V *out = (tail ? (V *)a.racc : fout) + cb;
+    V *out = fout + cb;
 #pragma unroll
     for (int k = 0; k < KC; k++) {
       const int comp = w + 8 * k;
