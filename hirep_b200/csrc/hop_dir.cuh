@@ -185,7 +185,9 @@ __global__ void __launch_bounds__(HD_THREADS, MINB) k_hop_dir(HopArgs<R> a) {
   V ax[KC], rr[KC];
   V co[EP == EP_AXPY ? 1 : KO];
   R cd[KC];
-  const bool use_aux = EP == EP_CLOV || (EP == EP_AXPY && a.aux != nullptr && a.caux != (R)0);
+  const bool axpy = EP == EP_AXPY && a.aux != nullptr && a.caux != (R)0;
+  // the inverters' <gamma_5 aux, result> needs aux whether or not it enters the result (m = -4)
+  const bool use_aux = EP == EP_CLOV || axpy || (EP == EP_AXPY && a.red_g5);
   auto load_epilogue = [&]() {
 #pragma unroll
     for (int k = 0; k < KC; k++)
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(HD_THREADS, MINB) k_hop_dir(HopArgs<R> a) {
       }
       r = cscale(ca, r);
       if constexpr (EP == EP_AXPY) {
-        if (use_aux) rmac(r, a.caux, ax[k]);
+        if (axpy) rmac(r, a.caux, ax[k]);
       }
       acc[k] = r;
     }

@@ -109,3 +109,30 @@ def test_g5qmr_forms(op, par, variant, pin):
         for s, x in zip(shifts, outs):
             xh = x.download()
             assert np.linalg.norm(b - (apply(m, xh) - s * xh)) < 1.1e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("variant", [0, 1, 4])
+@pytest.mark.parametrize("ng,rep", GROUPS)
+def test_g5qmr_without_a_diagonal_term(ng, rep, variant, pin):
+    """m = -4: the operator has no diagonal term, but the inverter's product with its input stays."""
+    o, lat = setup(ng, rep, (4, 6, 2, 4))
+    if variant == 4 and o.nf > 4:
+        pytest.skip("variant 4 is built for NF <= 4")
+    m = -4.0
+    o.set_mass(m)
+    pin(variant)
+    b = F.gaussian_spinor(4, o.VH, o.nf)
+    fb = lat.field(G.EVEN, host=b)
+    # the hops have norm at most 4 each: the shifted systems have condition numbers of at most 3
+    for shifts in ([40.0], [32.0, 40.0, -33.0]):
+        outs = [lat.field(G.EVEN) for _ in shifts]
+        if len(shifts) == 1:
+            lat.la("zero", outs[0])
+        it, ok = lat.g5QMR_mshift(G.OP_DPHI_EOPRE, m, shifts, 1e-20, fb, outs)
+        xo, it_o = o.g5QMR_mshift(G.OP_DPHI_EOPRE, shifts, 1e-20, b)
+        # the same recursion (a stopping test within rounding of its limit may fall either way)
+        assert ok and abs(it - it_o) <= 1, (it, it_o)
+        for s, x, y in zip(shifts, outs, xo):
+            xh = x.download()
+            assert np.linalg.norm(b - (o.Dphi_eopre(m, xh) - s * xh)) < 1.1e-10 * np.linalg.norm(b)
+            assert np.linalg.norm(xh - y) < 1e-9 * np.linalg.norm(y)
