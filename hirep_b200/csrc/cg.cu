@@ -33,6 +33,7 @@ constexpr int CG_HARD_LIMIT = 200000;  // iterations, when the caller sets no ma
 struct CGState {
   double omega, oldomega, gamma, alpha, lambda, delta, innorm2, err2;
   int n, state, iter, max_iter, notconv, flt;
+  int bad;  // <k, Mk> was zero or not finite (k_cg_fold_alpha; k_cg_fold_lambda ends the solve)
   double shift[MAXS], z1[MAXS], z2[MAXS], z3[MAXS];
   int flag[MAXS];
   // the last iterations' coefficients of the shifted systems, not yet applied to the fields:
@@ -60,16 +61,14 @@ __device__ double fold_partials(const double *partials, int nblocks, int stride)
 }
 
 // alpha = <k, Mk>; omega = -delta/alpha; z3 and the solution coefficients
-// (cg_mshift.c:82-91), one thread per shift.  The first kernel of an iteration to
-// change the state: an iteration after the one that converged only marks the end.
+// (cg_mshift.c:82-91), one thread per shift.  It may run beside the first hop of the second
+// H, whose threads read the state to decide whether to leave ahead of a barrier, so it only
+// reads the state and leaves a breakdown in bad.
 // slot: the iteration's place among those kept for the shifted systems.
 __global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_alpha(CGState *S, const double *partials, int nblocks, int stride,
                                                                 int slot) {
   if (slot == 0 && threadIdx.x == 0) S->pend = 0;
-  if (S->state != 0) {
-    if (threadIdx.x == 0 && S->state == 1) S->state = 2;
-    return;
-  }
+  if (S->state != 0) return;
   const double alpha = fold_partials(partials, nblocks, stride);
   const bool bad = !isfinite(alpha) || alpha == 0.0;  // breakdown (non-positive operator or NaN input)
   const double omega = -S->delta / alpha, oldomega = S->omega, gamma = S->gamma;
@@ -87,19 +86,26 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_alpha(CGState *S, cons
   __syncthreads();
   if (i == 0) {
     S->alpha = alpha;
-    if (bad) {
-      S->state = 3;
-    } else {
+    S->bad = bad;
+    if (!bad) {
       S->oldomega = oldomega;
       S->omega = omega;
     }
   }
 }
 
-// lambda = |r|^2, gamma, convergence flags (cg_mshift.c:92-111; cg_mshift_flt.c:96-118)
+// lambda = |r|^2, gamma, convergence flags (cg_mshift.c:92-111; cg_mshift_flt.c:96-118).
+// The only kernel that changes the state, when nothing runs beside it: 1 in the iteration that
+// converged, whose updates still follow, 2 in the one after it, 3 in one that broke down
+// (its residual, made with the iteration before's omega, is not used).
 __global__ void __launch_bounds__(FOLD_THREADS) k_cg_fold_lambda(CGState *S, const double *partials, int nblocks, int slot) {
   pdl_enter();
-  if (S->state != 0) return;
+  const int state = S->state, bad = S->bad;
+  __syncthreads();
+  if (state != 0 || bad) {
+    if (threadIdx.x == 0) S->state = state == 0 ? 3 : (state == 1 ? 2 : state);
+    return;
+  }
   const double lambda = fold_partials(partials, nblocks, 1);
   const double gamma = lambda / S->delta;
   const int i = threadIdx.x;

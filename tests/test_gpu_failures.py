@@ -85,6 +85,42 @@ def test_singular_system_is_a_breakdown():
     assert status_of(e.value) == G.E_BREAKDOWN
 
 
+@pytest.mark.parametrize("variant", [-1, 0, 1, 2, 4])
+@pytest.mark.parametrize("shifts", [[0.0], [0.0, -1.0, -3.0]])
+@pytest.mark.parametrize("flt", [False, True])
+@pytest.mark.parametrize("clover", [False, True])
+def test_breakdown_in_captured_iterations(clover, flt, shifts, variant):
+    """The same singular system once the hopping kernels are tuned, so that its iterations
+    are captured as a graph (where alpha is folded beside a hop): the breakdown ends the
+    solve in its first iteration and leaves nothing behind for the next one."""
+    lat = unit_lattice()
+    lib = G.lib()
+    op = G.OP_G5CPHI_EOPRE_SQ if clover else G.OP_G5DPHI_EOPRE_SQ
+    if clover:
+        lat.clover_init(1.0)  # the clover term of unit links is zero: D = 4 + m
+    fin = lat.field(G.EVEN, host=ones(lat))
+    xs = [lat.field(G.EVEN) for _ in shifts]
+    try:
+        G._check(lib.hrgpu_set_hop_variant(variant), "set_hop_variant")
+        for _ in range(2):
+            # m = -2 (Wilson) or 4 (clover): D_eo D_oe psi = 16 psi, so H psi = (4 - 16) g5 psi
+            # or (8 - 16/8) g5 psi, and H^2 psi = 144 psi or 36 psi
+            m, ev = (4.0, 36.0) if clover else (-2.0, 144.0)
+            lat.la("zero", xs[0])
+            _, ok = lat.cg_mshift(op, m, shifts, 1e-24, fin, xs, max_iter=200, flt=flt)
+            assert ok
+            for s, x in zip(shifts, xs):
+                # the residual's elements are all alike: |r| <= sqrt(err2) |b| holds for each
+                assert np.abs(x.download() - ones(lat) / (ev - s)).max() < 1.01e-12 / (ev - s)
+            lat.la("zero", xs[0])
+            with pytest.raises(G.HRGPUError, match=r"breakdown at iteration [01] ") as e:
+                lat.cg_mshift(op, 0.0, shifts, 1e-24, fin, xs, max_iter=200, flt=flt)
+            assert status_of(e.value) == G.E_BREAKDOWN
+            assert all(not np.any(x.download()) for x in xs)
+    finally:
+        lib.hrgpu_set_hop_variant(-1)
+
+
 def test_shift_on_an_eigenvalue_is_a_breakdown():
     """m0 = -2: H^2 psi = 144 psi exactly; the multi-shift solve of (H^2 - s) for
     s = 0 and s = 144 must not report success for the singular second system."""
