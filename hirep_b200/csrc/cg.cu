@@ -261,6 +261,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_dot(const CGState *S, const 
 // ---------------------------------------------------------------------------
 // workspace (cached between calls, grown on demand)
 // ---------------------------------------------------------------------------
+// The padding of the work fields (components are L.ld >= VH sites apart) is kept at zero: the
+// hops write the sites alone, but the updates and the norms run over whole fields.
 struct CGWork {
   std::vector<void *> bufs;  // p[0..n-1], k, r, Mk, and where memory allows CG_CHUNK - 1 more residuals
   size_t bytes = 0;
@@ -290,6 +292,7 @@ static int cg_workspace(int prec, int nvec, size_t bytes) {
     void *b = nullptr;
     HR_CUDA(cudaMalloc(&b, bytes));
     w.bufs.push_back(b);
+    HR_CUDA(cudaMemsetAsync(b, 0, bytes, L.stream));
   }
   if (!w.S) {
     HR_CUDA(cudaMalloc(&w.S, sizeof(CGState)));
@@ -309,6 +312,11 @@ static bool cg_more_residuals(CGWork &w, int nvec) {
     if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail / 2 < (CG_CHUNK - 1) * w.bytes ||
         cudaMalloc(&b, w.bytes) != cudaSuccess) {
       cudaGetLastError();
+      return false;
+    }
+    if (cudaMemsetAsync(b, 0, w.bytes, L.stream) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(b);
       return false;
     }
     w.bufs.push_back(b);
@@ -633,7 +641,13 @@ static int cg_core(int op, double mass, int n, const double *shift, double err2,
   if (rc) return rc;
   const CGState &h = w.hS[cur];
   cgiter += h.iter;
+  // coefficients that were not finite may have reached the padding
+  auto clear_padding = [&]() -> int {
+    for (void *b : w.bufs) HR_CUDA(cudaMemsetAsync(b, 0, bytes, L.stream));
+    return 0;
+  };
   if (h.state == 3) {
+    if (int q = clear_padding()) return q;
     *iters = cgiter;
     set_error("cg_mshift: breakdown at iteration %d (alpha=%g, |r|^2=%g)", cgiter, h.alpha, h.lambda);
     return HRGPU_E_BREAKDOWN;
@@ -648,6 +662,7 @@ static int cg_core(int op, double mass, int n, const double *shift, double err2,
       double nr;
       if (int q = la_dot(2, par, prec, Mk, nullptr, &nr)) return q;
       if (!isfinite(nr)) {
+        if (int q = clear_padding()) return q;
         *iters = cgiter;
         set_error("cg_mshift: the true residual of shift %d is not finite (%g)", i, nr);
         return HRGPU_E_BREAKDOWN;
@@ -713,6 +728,7 @@ int hrgpu_cg_mshift_flt(int op, double mass, int n, const double *shift, double 
     HR_CUDA(cudaMalloc(&FW.dres, bd));
     HR_CUDA(cudaMalloc(&FW.dres2, bd));
     HR_CUDA(cudaMalloc(&FW.dtmp, bd));
+    for (void *b : {FW.dres, FW.dres2, FW.dtmp}) HR_CUDA(cudaMemsetAsync(b, 0, bd, L.stream));
     FW.bd = bd;
   }
   if (FW.bf != bf) {
@@ -724,6 +740,7 @@ int hrgpu_cg_mshift_flt(int op, double mass, int n, const double *shift, double 
     void *b;
     HR_CUDA(cudaMalloc(&b, bf));
     FW.fbuf.push_back(b);
+    HR_CUDA(cudaMemsetAsync(b, 0, bf, L.stream));
   }
   void *dres = FW.dres, *dres2 = FW.dres2, *dtmp = FW.dtmp;
   std::vector<void *> &fbuf = FW.fbuf;

@@ -3,6 +3,7 @@ at every place among those, with shifts that converge in different iterations, i
 and with the FP32 inner solve, against the oracle's solutions and iteration counts."""
 import numpy as np
 import pytest
+import torch
 
 import oracle as O
 from hirep_b200 import fields as F
@@ -68,3 +69,27 @@ def test_shifts_inner_solve_in_fp32():
             xh = x.download()
             r = b - (o.g5Cphi_eopre_sq(M, xh) - s * xh)
             assert np.linalg.norm(r) ** 2 < 1.01 * err2 * np.linalg.norm(b) ** 2
+
+
+@pytest.mark.parametrize("flt", [False, True])
+@pytest.mark.parametrize("ng,rep", [(3, O.FUND), (4, O.ASYM)])
+def test_padding_stays_zero(ng, rep, flt):
+    """The parities of these lattices are no multiple of the 32 sites that a field's components
+    are padded to.  The library's workspaces are made of memory that the solve before has left
+    full of numbers (another lattice, then another size of field); none of them may get into the
+    padding of a solution, which the norms run over."""
+    for dims in ((8, 8, 8, 8), (6, 4, 2, 10), (4, 6, 6, 14), (4, 2, 6, 2)):
+        lat = G.Lattice(*dims, ng, rep)
+        lat.set_gauge(F.smooth_gauge(5, lat.V, ng, 0.3))
+        lat.represent_gauge_field(True)
+        pad = (-lat.VH) % 32
+        for op, par, n in ((G.OP_G5DPHI_SQ, G.FULL, 1), (G.OP_G5DPHI_EOPRE_SQ, G.EVEN, 10),
+                           (G.OP_G5DPHI_SQ, G.FULL, 3), (G.OP_G5DPHI_EOPRE_SQ, G.EVEN, 1)):
+            b = lat.field(par, host=F.gaussian_spinor(3, lat.nsites(par), lat.nf))
+            outs = [lat.field(par) for _ in range(n)]
+            it, ok = lat.cg_mshift(op, M, [0.0, *(-float(10.0 ** (k - 6)) for k in range(9))][:n], 1e-20, b, outs, flt=flt)
+            assert ok
+            for x in outs:
+                v = x.buf.view(torch.float64).view(2 if par == G.FULL else 1, 4 * lat.nf, -1, 2)
+                assert v.shape[2] == lat.VH + pad
+                assert not v[:, :, lat.VH:].any(), (dims, op, n)
