@@ -83,18 +83,15 @@ static inline void (*hop_kernel(int recon, bool tail))(HopArgs<R>) {
 }
 
 // variant 1: one warp per direction (k_hop_dir) for NF <= 6, two threads per site
-// (k_hop2) for larger NF.  Links are rebuilt or built from the fundamental ones where
-// variants 0 and 6 would do so.
+// (k_hop2) for larger NF.  Links are built from the fundamental ones where variant 6
+// would do so.
 template <int N, bool RL, typename R, int EP, typename LE = typename LinkE<RL, R>::T>
 int launch_dir(HopArgs<R> &a, long nsites, cudaStream_t s) {
   if constexpr (HopDirOK<N>::v) {
     constexpr bool stored = std::is_same<LE, typename LinkE<RL, R>::T>::value;  // not BF16
     void (*f)(HopArgs<R>) = k_hop_dir<N, RL, R, EP, 2, LE>;
-    if constexpr (stored && N == 3) {
-      if (a.recon) f = k_hop_dir<N, RL, R, EP, 2, LE, true>;
-    }
     if constexpr (stored && N == 6 && !RL) {
-      if (a.recon >= 3 && a.Ug) f = L.repr == HRGPU_SYM ? k_hop_dir<N, RL, R, EP, 2, LE, false, 1> : k_hop_dir<N, RL, R, EP, 2, LE, false, 2>;
+      if (a.recon >= 3 && a.Ug) f = L.repr == HRGPU_SYM ? k_hop_dir<N, RL, R, EP, 2, LE, 1> : k_hop_dir<N, RL, R, EP, 2, LE, 2>;
     }
     constexpr int smem = HopDirLayout<N, R, EP>::SMEM;
     if (smem > 40 * 1024)  // with the static part of the norm's sum, at NF = 6
