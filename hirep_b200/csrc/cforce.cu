@@ -22,7 +22,9 @@
 // site (Z is read once), k_cforce_plaq carries the seven that a plaquette needs to
 // its links, one thread per (plaquette, plane), and k_cforce_gather adds the six
 // contributions to each link in a fixed order, so the result does not depend on
-// scheduling.
+// scheduling.  The corners and link forces take 42 NG^2 + 24 (NG^2 - 1) doubles per site
+// (3.0 GB for SU(3) at 48x24^3), kept for the next force; they are only taken where
+// as much again stays free.
 #include "suN.cuh"
 
 namespace hrgpu {
@@ -277,7 +279,8 @@ int clover_force_fund(double coeff, int **bad_out) {
   const long lp = 2L * L.ld;
   const int N2 = L.ng * L.ng;
   const size_t nc = (size_t)6 * CF_SLOTS * N2 * lp, nf = (size_t)24 * L.dimg * lp;  // corners, link forces
-  if (!L.cl_plaq && cudaMalloc(&L.cl_plaq, sizeof(double) * (nc + nf + 1)) != cudaSuccess) {
+  const size_t bytes = sizeof(double) * (nc + nf + 1);
+  if (!L.cl_plaq && (!optional_room(bytes) || cudaMalloc(&L.cl_plaq, bytes) != cudaSuccess)) {
     cudaGetLastError();  // no room for the workspace: the representation's kernel needs none
     L.cl_plaq = nullptr;
     return -1;

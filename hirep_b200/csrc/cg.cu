@@ -306,11 +306,11 @@ static int cg_workspace(int prec, int nvec, size_t bytes) {
 // CG_CHUNK - 1 more residuals behind the first nvec fields, where they leave as much again
 // free: true if they are there.  Without them the solve runs as well, updating every iteration.
 static bool cg_more_residuals(CGWork &w, int nvec) {
+  if (!optional_allowed()) return false;
   while ((int)w.bufs.size() < nvec + CG_CHUNK - 1) {
-    size_t avail = 0, total = 0;
     void *b = nullptr;
-    if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail / 2 < (CG_CHUNK - 1) * w.bytes ||
-        cudaMalloc(&b, w.bytes) != cudaSuccess) {
+    if (!optional_room((CG_CHUNK - 1) * w.bytes)) return false;
+    if (cudaMalloc(&b, w.bytes) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
@@ -349,6 +349,17 @@ static void drop_cg_graph(CGGraph &c) {
   c = CGGraph();
 }
 
+void cg_drop_work() {
+  for (int q = 0; q < 2; q++) {
+    for (cudaEvent_t ev : W[q].ev)  // a solve leaves a chunk in flight behind its last one
+      if (ev) cudaEventSynchronize(ev);
+    drop_cg_graph(CGG[q]);
+    for (void *b : W[q].bufs) cudaFree(b);
+    W[q].bufs.clear();
+    W[q].bytes = 0;
+  }
+}
+
 void cg_release() {
   batch_release();
   qmr_release();
@@ -357,7 +368,7 @@ void cg_release() {
   cudaFree(FW.dres); cudaFree(FW.dres2); cudaFree(FW.dtmp);
   for (void *b : FW.fbuf) cudaFree(b);
   FW = FltWork();
-  for (int q = 0; q < 2; q++) drop_cg_graph(CGG[q]);
+  cg_drop_work();
   if (cg_cap) cudaStreamDestroy(cg_cap);
   if (cg_cap2) cudaStreamDestroy(cg_cap2);
   for (cudaEvent_t &ev : cg_ev) {
@@ -366,9 +377,6 @@ void cg_release() {
   }
   cg_cap = cg_cap2 = nullptr;
   for (int q = 0; q < 2; q++) {
-    for (void *b : W[q].bufs) cudaFree(b);
-    W[q].bufs.clear();
-    W[q].bytes = 0;
     if (W[q].S) cudaFree(W[q].S);
     if (W[q].hS) cudaFreeHost(W[q].hS);
     for (cudaEvent_t &ev : W[q].ev) {

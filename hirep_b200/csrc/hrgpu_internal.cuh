@@ -149,6 +149,11 @@ inline size_t spinor_bytes(int par, int prec) {
 }
 
 int ensure_tmp(void **p, size_t bytes);
+// whether a workspace may be taken that only a faster path needs (hrgpu_set_optional_workspace):
+// it must leave as much again free for the fields, which have no path without
+bool optional_room(size_t bytes);
+bool optional_allowed();
+void cg_drop_work();  // the CG's work fields
 int library_device();  // the device of hrgpu_init (-1 before)
 int ensure_links_bf16();  // the BF16 copy of the links, made from the FP64 ones when they changed
 int detect_recon12();     // check links set already represented for row-2 reconstruction

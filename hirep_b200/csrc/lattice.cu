@@ -39,6 +39,18 @@ int ensure_tmp(void **p, size_t bytes) {
   return 0;
 }
 
+static bool g_optional = true;
+bool optional_allowed() { return g_optional; }
+bool optional_room(size_t bytes) {
+  size_t avail = 0, total = 0;
+  if (!g_optional) return false;
+  if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return avail / 2 >= bytes;
+}
+
 int ensure_stage(size_t bytes) {
   if (L.stage_bytes >= bytes) return 0;
   if (L.stage) HR_CUDA(cudaFree(L.stage));
@@ -663,6 +675,17 @@ int hrgpu_gauge_set(const double *u_host) {
   fund_links_changed();
   HR_CUDA(cudaStreamSynchronize(L.stream));
   L.have_fund = true;
+  return 0;
+}
+
+int hrgpu_set_optional_workspace(int on) {
+  HR_REQUIRE(on == 0 || on == 1, HRGPU_E_ARG, "set_optional_workspace: on must be 0 or 1");
+  g_optional = on != 0;
+  if (!on) {
+    if (L.cl_plaq) HR_CUDA(cudaFree(L.cl_plaq));
+    L.cl_plaq = nullptr;
+    cg_drop_work();
+  }
   return 0;
 }
 

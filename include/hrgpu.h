@@ -86,6 +86,11 @@ size_t hrgpu_spinor_bytes(int par, int prec);
  * Until this is called the library uses a stream of its own. */
 int hrgpu_set_stream(void *cuda_stream);
 int hrgpu_synchronize(void);
+/* 1 (default): workspaces that only a faster path needs (the clover force's,
+ * 42 NG^2 + 24 (NG^2 - 1) doubles per site, and three residuals of the multi-shift CG)
+ * are taken on first use where as much again stays free, and kept.  0: they are given
+ * back, with the CG's work fields, and the paths without them run. */
+int hrgpu_set_optional_workspace(int on);
 
 /* --------------------------------------------------------- gauge fields -- */
 /* u_gauge upload (Include/global.h:143, HiRep layout [V][4][NG*NG] complex) */
