@@ -38,7 +38,7 @@ def test_ends_of_a_solve(ng, rep, op, par, clover):
     b = F.gaussian_spinor(3, lat.nsites(par), o.nf)
     fb = lat.field(par, host=b)
     for n in (1, 2, 5):
-        ends = set()
+        ends, other = set(), 0
         for e in range(4, 16):
             err2 = 10.0 ** -e
             outs = [lat.field(par) for _ in range(n)]
@@ -46,14 +46,16 @@ def test_ends_of_a_solve(ng, rep, op, par, clover):
                 lat.la("zero", outs[0])
             it, ok = lat.cg_mshift(op, M, shifts[:n], err2, fb, outs)
             xo, it_o = o.cg_mshift(op, shifts[:n], err2, b)
-            assert ok
-            if it == it_o:  # (a stopping test within rounding of its limit may fall either way)
+            # a stopping test within rounding of its limit may fall either way
+            assert ok and abs(it - it_o) <= 1, (n, err2, it, it_o)
+            other += it != it_o
+            if it == it_o:
                 ends.add((it - n) % 4)
                 # the same recursion in FP64: rounding of some tens of iterations times the
                 # condition number (below 1e3), far below one iteration's change (err2 >= 1e-15)
                 for x, y in zip(outs, xo):
                     assert np.linalg.norm(x.download() - y) < 1e-11 * np.linalg.norm(y), (n, err2)
-        assert len(ends) >= 3
+        assert len(ends) >= 3 and other <= 1
 
 
 def test_shifts_inner_solve_in_fp32():
