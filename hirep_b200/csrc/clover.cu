@@ -638,7 +638,7 @@ int compute_clover_term_dev() {
 template <int N>
 static int launch_pack(double sigma) {
   if constexpr (N <= 6) {
-    HR_CUDA(cudaFuncSetAttribute(k_clover_pack<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pack<N>::SMEM));
+    if (int rc = allow_smem((const void *)k_clover_pack<N>, Pack<N>::SMEM)) return rc;
     k_clover_pack<N><<<(unsigned)(2L * L.ld / PK_S), Pack<N>::TH, Pack<N>::SMEM, L.stream>>>(
         L.cl_term, sigma, L.cl_dg, L.cl_od, L.cl_idg, L.cl_iod, L.cl_ldet, make_geo());
   }

@@ -117,7 +117,7 @@ static int launch_term(const double2 *Ul) {
   constexpr int NF = Rep<NG, RP>::NF;
   constexpr int smem = (int)sizeof(double) * 6 * NF * NF * 32;
   if (smem > 48 * 1024)
-    HR_CUDA(cudaFuncSetAttribute(k_clover_term_fund<NG, RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (int rc = allow_smem((const void *)k_clover_term_fund<NG, RP>, smem)) return rc;
   k_clover_term_fund<NG, RP><<<(unsigned)(2L * L.ld / 32), 192, smem, L.stream>>>(L.cl_term, Ul, make_geo(), L.csw);
   HR_LAUNCH_CHECK();
   return 0;

@@ -842,7 +842,7 @@ template <int N, bool REAL>
 static int launch_clover_fermion(const double2 *X, const double2 *Y, Geo g, double residue) {
   constexpr int smem = (int)sizeof(double2) * 8 * N * 32;
   if (smem > 48 * 1024)
-    HR_CUDA(cudaFuncSetAttribute(k_force_clover_fermion<N, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (int rc = allow_smem((const void *)k_force_clover_fermion<N, REAL>, smem)) return rc;
   k_force_clover_fermion<N, REAL><<<(unsigned)(2L * g.ld / 32), 192, smem, L.stream>>>(L.cl_force, X, Y, g, residue,
                                                                                    !L.cl_force_zero);
   L.cl_force_zero = false;

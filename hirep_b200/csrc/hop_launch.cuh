@@ -95,7 +95,7 @@ int launch_dir(HopArgs<R> &a, long nsites, cudaStream_t s) {
     }
     constexpr int smem = HopDirLayout<N, R, EP>::SMEM;
     if (smem > 40 * 1024)  // with the static part of the norm's sum, at NF = 6
-      HR_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      if (int rc = allow_smem((const void *)f, smem)) return rc;
     const dim3 grid((unsigned)((nsites + HD_SITES - 1) / HD_SITES), a.both ? 2 : 1);
     HR_CUDA(launch_pdl<R>(f, grid, dim3(HD_THREADS), smem, s, a, true));
   } else {

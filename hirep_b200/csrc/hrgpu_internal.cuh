@@ -154,6 +154,8 @@ int ensure_tmp(void **p, size_t bytes);
 bool optional_room(size_t bytes);
 bool optional_allowed();
 void cg_drop_work();  // the CG's work fields
+// a kernel's limit of dynamic shared memory raised, once per kernel and device
+int allow_smem(const void *kernel, int bytes);
 int library_device();  // the device of hrgpu_init (-1 before)
 int ensure_links_bf16();  // the BF16 copy of the links, made from the FP64 ones when they changed
 int detect_recon12();     // check links set already represented for row-2 reconstruction

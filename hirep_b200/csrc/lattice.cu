@@ -4,6 +4,8 @@
 #include <string.h>
 
 #include <complex>
+#include <set>
+#include <utility>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -36,6 +38,15 @@ int ensure_tmp(void **p, size_t bytes) {
   if (*p) return 0;
   HR_CUDA(cudaMalloc(p, bytes));
   HR_CUDA(cudaMemsetAsync(*p, 0, bytes, L.stream));
+  return 0;
+}
+
+int allow_smem(const void *kernel, int bytes) {
+  static std::set<std::pair<const void *, int>> done;
+  const std::pair<const void *, int> key(kernel, g_device);
+  if (done.count(key)) return 0;
+  HR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  done.insert(key);
   return 0;
 }
 
