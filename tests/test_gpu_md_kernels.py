@@ -82,6 +82,19 @@ def test_clover_force(ng, rep, dims, exp):
     assert np.abs(got - ref).max() < 2e-13 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("off", [0.0, 1e-14, 4e-13])
+@pytest.mark.parametrize("ng,rep", [(3, O.FUND), (3, O.SYM), (4, O.ASYM)])
+def test_clover_force_on_links_that_are_nearly_unitary(ng, rep, off):
+    """A scale factor 1 + off in every link: the force is the reference's for the links as they are."""
+    o, lat, u, _ = setup(ng, (4, 2, 2, 4), rep)
+    u = u * (1.0 + off)
+    o.set_gauge(o.represent_gauge_field(u, True))
+    lat.set_gauge(u)
+    lat.represent_gauge_field(True)
+    got, ref = clover_force_pair(o, lat, False)
+    assert np.abs(got - ref).max() < 2e-13 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("uploaded", [False, True])
 def test_clover_force_in_the_representation(uploaded):
     """Links that are not unitary, and represented links uploaded by themselves."""
