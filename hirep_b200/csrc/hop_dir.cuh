@@ -75,15 +75,14 @@ __device__ __forceinline__ void hd_mac(double2 &a, double u, double2 h) { rmac(a
 template <bool DAG>
 __device__ __forceinline__ void hd_mac(float2 &a, float u, float2 h) { rmac(a, u, h); }
 
-// A link as it is read: NF x NF stored elements, or the fundamental link (FR); loaded early
-// where it fits in registers beside a neighbour's spinor.  (Row 2 of a 3 x 3 link is not
-// rebuilt here as in k_hop: these lattices lie in L2, where it saves nothing, and its
-// roundings raised the operator's error at 8^4 from 1.04e-16 to 1.36e-16.)
-template <int NFT, bool REAL, typename R, typename LE, int FR>
+// A link as it is read: NF x NF stored elements, rows 0 and 1 (RC), or the fundamental
+// link (FR); loaded early where it fits in registers beside a neighbour's spinor.
+template <int NFT, bool REAL, typename R, typename LE, bool RC, int FR>
 struct HdLink {
   typedef typename C2<R>::T V;
   static constexpr bool bf16 = std::is_same<LE, __nv_bfloat162>::value || std::is_same<LE, __nv_bfloat16>::value;
   static constexpr int NG = FR ? TwoIdx<FR ? FR : 1>::NG : 0;
+  static constexpr bool rc = RC && NFT == 3 && !bf16;
   static constexpr int NE = FR ? NG * NG : NFT * NFT;
   static constexpr bool EARLY = NE <= 16;
   typedef typename std::conditional<FR != 0, V, typename std::conditional<bf16, typename std::conditional<REAL, R, V>::type, LE>::type>::type E;
@@ -101,10 +100,20 @@ struct HdLink {
       sg = (a.recon == 4 && flip) ? (R)-1 : (R)1;
     } else {
       U = (const LE *)a.U + (long)mu * NFT * NFT * plane + site;
-      if constexpr (EARLY) {
+      if constexpr (rc) {
+#pragma unroll
+        for (int e = 0; e < 6; e++) u[e] = ld_u(U + (long)e * plane);
+        sg = (a.recon == 2 && flip) ? (R)-1 : (R)1;
+      } else if constexpr (EARLY) {
 #pragma unroll
         for (int e = 0; e < NE; e++) u[e] = hd_elem(U + (long)e * plane);
       }
+    }
+  }
+  __device__ __forceinline__ void ready() {
+    if constexpr (rc) {
+      if constexpr (REAL) so3_row2(u, sg);
+      else su3_row2(u, sg);
     }
   }
   __device__ __forceinline__ E operator()(int i, int j) const {
@@ -131,7 +140,8 @@ __device__ __forceinline__ void hd_link(const LK &link, V *c0, V *c1, const V (&
   }
 }
 
-template <int NFT, bool REAL, typename R, int EP, int MINB, typename LE = typename LinkE<REAL, R>::T, int FR = 0>
+template <int NFT, bool REAL, typename R, int EP, int MINB, typename LE = typename LinkE<REAL, R>::T, bool RC = false,
+          int FR = 0>
 __global__ void __launch_bounds__(HD_THREADS, MINB) k_hop_dir(HopArgs<R> a) {
   typedef typename C2<R>::T V;
   typedef HopDirLayout<NFT, R, EP> LAY;
@@ -166,7 +176,7 @@ __global__ void __launch_bounds__(HD_THREADS, MINB) k_hop_dir(HopArgs<R> a) {
   const int cn = coords_to_cb(g, t, x, y, z);
   const long site = (long)outp * ld + cb;
   if (!a.pre) pdl_enter();
-  typedef HdLink<NFT, REAL, R, LE, FR> LK;
+  typedef HdLink<NFT, REAL, R, LE, RC, FR> LK;
   LK link;
   link.load(a, mu, bw ? (long)inp * ld + cn : site, flip);
   // what the epilogue reads from memory: with the link where the registers allow it,
@@ -213,6 +223,7 @@ __global__ void __launch_bounds__(HD_THREADS, MINB) k_hop_dir(HopArgs<R> a) {
       else { h0[i] = caddi(s0, p0); h1[i] = csubi(s1, p1); }
     }
     V *c0 = sc + (long)(2 * w) * NFT * HD_SITES + lane, *c1 = c0 + NFT * HD_SITES;
+    link.ready();
     if (!bw) hd_link<NFT, false>(link, c0, c1, h0, h1);
     else hd_link<NFT, true>(link, c0, c1, h0, h1);
   }

@@ -84,14 +84,20 @@ static inline void (*hop_kernel(int recon, bool tail))(HopArgs<R>) {
 
 // variant 1: one warp per direction (k_hop_dir) for NF <= 6, two threads per site
 // (k_hop2) for larger NF.  Links are built from the fundamental ones where variant 6
-// would do so.
+// would do so.  Row 2 of a 3 x 3 link is rebuilt in FP32 only: in FP64 that saves nothing on
+// the lattices that lie in L2, and its roundings raised the operator's error at 8^4 from
+// 1.0e-16 to 1.3e-16; in FP32, whose operator the variants 0 and 2 apply with rebuilt rows as
+// well, it takes 7.8 us instead of 11.5 on 10x14x12x20.
 template <int N, bool RL, typename R, int EP, typename LE = typename LinkE<RL, R>::T>
 int launch_dir(HopArgs<R> &a, long nsites, cudaStream_t s) {
   if constexpr (HopDirOK<N>::v) {
     constexpr bool stored = std::is_same<LE, typename LinkE<RL, R>::T>::value;  // not BF16
     void (*f)(HopArgs<R>) = k_hop_dir<N, RL, R, EP, 2, LE>;
+    if constexpr (stored && N == 3 && sizeof(R) == 4) {
+      if (a.recon) f = k_hop_dir<N, RL, R, EP, 2, LE, true>;
+    }
     if constexpr (stored && N == 6 && !RL) {
-      if (a.recon >= 3 && a.Ug) f = L.repr == HRGPU_SYM ? k_hop_dir<N, RL, R, EP, 2, LE, 1> : k_hop_dir<N, RL, R, EP, 2, LE, 2>;
+      if (a.recon >= 3 && a.Ug) f = L.repr == HRGPU_SYM ? k_hop_dir<N, RL, R, EP, 2, LE, false, 1> : k_hop_dir<N, RL, R, EP, 2, LE, false, 2>;
     }
     constexpr int smem = HopDirLayout<N, R, EP>::SMEM;
     if (smem > 40 * 1024)  // with the static part of the norm's sum, at NF = 6

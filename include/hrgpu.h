@@ -102,8 +102,8 @@ int hrgpu_represent_gauge_field(int bc_t_antiperiodic);
 /* SU(3) fundamental and SU(2) adjoint links: after represent_gauge_field has
  * checked that every link's row 2 equals s conj(r0 x r1) (adjoint: s (r0 x r1))
  * to 1e-14 (s = -1 on the links with the antiperiodic time sign), the
- * single-field hopping kernels of variants 0 and 2 load rows 0 and 1 only and
- * rebuild row 2 (the others read the full links).
+ * single-field hopping kernels of variants 0 and 2, and in FP32 of variant 1, load
+ * rows 0 and 1 only and rebuild row 2 (the others read the full links).
  * hrgpu_gauge_set_f runs the same check, trying the antiperiodic sign first.
  * The SU(3) symmetric and SU(4) antisymmetric representations (NF = 6): after
  * represent_gauge_field the single-field hopping kernel of variant 6 may

@@ -140,8 +140,8 @@ def test_g5qmr_without_a_diagonal_term(ng, rep, variant, pin):
 
 @pytest.mark.parametrize("ng,rep", [(3, O.FUND), (2, O.ADJ)])
 def test_reads_the_stored_links(ng, rep, pin):
-    """Row 2 of a 3 x 3 link is not rebuilt (the other variants do where it saves traffic, at
-    a few roundings): the result is that of the stored links, bit for bit."""
+    """In FP64 row 2 of a 3 x 3 link is not rebuilt (the other variants do where it saves traffic,
+    at a few roundings): the result is that of the stored links, bit for bit."""
     o, lat = setup(ng, rep, (6, 4, 2, 10), True)
     assert lat.link_recon() in (1, 2)
     pin(1)
