@@ -336,7 +336,7 @@ struct CGGraph {
   int op = -1;
   double mass = 0;
   const void *ptrs[9 + CG_CHUNK] = {};
-  int v[3] = {-1, -1, -1}, force = -1, flt_links = -1, pdl = -1, recon = -1, one = -1, keep = -1;
+  int v[3] = {-1, -1, -1}, force = -1, flt_links = -1, pdl = -1, recon = -1, one = -1, keep = -1, both = -1;
   unsigned long mvm = 0;  // hop launches in one replay (the MVM counter)
   cudaGraphExec_t exec = nullptr;
 };
@@ -476,12 +476,7 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *con
   if (prec == HRGPU_FLOAT && L.flt_links == HRGPU_LINKS_BF16)
     if (int rc = ensure_links_bf16()) return rc;
   const int pi = prec == HRGPU_DOUBLE ? 0 : (L.flt_links == HRGPU_LINKS_BF16 ? 2 : 1);
-  const bool clover = op_is_clover(op);
-  const bool settled = L.hop_force >= 0 || (clover ? (L.hop_variant[pi][EP_CLOV] >= 0 &&
-                                                      (op == HRGPU_OP_G5CPHI_SQ || op == HRGPU_OP_CPHI ||
-                                                       L.hop_variant[pi][EP_CLOV_INV] >= 0))
-                                                   : L.hop_variant[pi][EP_AXPY] >= 0);
-  if (!settled) {  // tunes the hopping kernels
+  if (!op_tuned(op, prec)) {  // tunes the hopping kernels
     const unsigned long m0 = mvm_count();
     const int rc = cg_iterations<R>(op, prec, mass, w, k, r, keep, Mk, ne, g, one, nullptr);
     *mvm = mvm_count() - m0;
@@ -495,8 +490,9 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *con
   for (int c = 0; c < CG_CHUNK; c++) ptrs[9 + c] = r[c % keep];
   CGGraph &c = CGG[prec];
   const int recon = L.recon_allow ? L.recon12 : 0;
+  const int both = L.hop_both[pi][op_is_clover(op) ? EP_CLOV : EP_AXPY];
   bool same = c.exec && c.op == op && c.mass == mass && c.force == L.hop_force && c.flt_links == L.flt_links &&
-              c.pdl == (int)L.hop_pdl && c.recon == recon && c.one == one && c.keep == keep;
+              c.both == both && c.pdl == (int)L.hop_pdl && c.recon == recon && c.one == one && c.keep == keep;
   for (int i = 0; i < 3 && same; i++) same = c.v[i] == L.hop_variant[pi][i];
   for (int i = 0; i < 9 + CG_CHUNK && same; i++) same = c.ptrs[i] == ptrs[i];
   if (!same) {
@@ -535,6 +531,7 @@ static int cg_chunk(int op, int prec, double mass, CGWork &w, void *k, void *con
     c.recon = recon;
     c.one = one;
     c.keep = keep;
+    c.both = both;
     for (int i = 0; i < 3; i++) c.v[i] = L.hop_variant[pi][i];
     for (int i = 0; i < 9 + CG_CHUNK; i++) c.ptrs[i] = ptrs[i];
     c.mvm = dm;

@@ -74,30 +74,115 @@ template int hop<double>(int, void *, const void *, int, double, const void *, d
 template int hop<float>(int, void *, const void *, int, double, const void *, double, int, double *, const float *,
                         const float2 *, int, int, const HopTail *);
 
-static int last_hop_variant(int ep, int prec) {
-  const int pi = prec == HRGPU_DOUBLE ? 0 : (L.flt_links == HRGPU_LINKS_BF16 ? 2 : 1);
-  return L.hop_force >= 0 ? L.hop_force : L.hop_variant[pi][ep];
+static int tune_slot(int prec) { return prec == HRGPU_DOUBLE ? 0 : (L.flt_links == HRGPU_LINKS_BF16 ? 2 : 1); }
+
+static int last_hop_variant(int ep, int prec) { return L.hop_force >= 0 ? L.hop_force : L.hop_variant[tune_slot(prec)][ep]; }
+
+// whether candidates may be timed now: nothing is forced, and no stream capture is on
+static bool can_tune() {
+  if (L.hop_force >= 0) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(L.stream, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return cs == cudaStreamCaptureStatusNone;
 }
 
-// the hop onto both parities of a full field: one launch where the variant in use
-// takes both (a small lattice then fills twice the SMs), else one per parity
+// milliseconds of run() on the GPU: the launches queue up behind a delay, since they cost the
+// host as much as the hops of a small lattice take.  The events resolve half a microsecond, so
+// a short run is repeated more often.
+template <typename F>
+static int time_launches(F &&run, float *ms) {
+  cudaEvent_t e[2] = {nullptr, nullptr};
+  int rc = 0;
+  if (cudaEventCreate(&e[0]) != cudaSuccess || cudaEventCreate(&e[1]) != cudaSuccess)
+    rc = fail_cuda(cudaGetLastError(), "cudaEventCreate", __FILE__, __LINE__);
+  for (int reps = 3; !rc; reps = 10) {
+    rc = stream_delay(reps == 3 ? 30.0 : 80.0);
+    if (!rc) rc = run();
+    if (!rc && cudaEventRecord(e[0], L.stream) != cudaSuccess) rc = fail_cuda(cudaGetLastError(), "cudaEventRecord", __FILE__, __LINE__);
+    for (int r = 0; r < reps && !rc; r++) rc = run();
+    if (!rc && (cudaEventRecord(e[1], L.stream) != cudaSuccess || cudaEventSynchronize(e[1]) != cudaSuccess ||
+                cudaEventElapsedTime(ms, e[0], e[1]) != cudaSuccess))
+      rc = fail_cuda(cudaGetLastError(), "hop timing", __FILE__, __LINE__);
+    *ms /= reps;
+    if (reps > 3 || *ms > 0.05f) break;
+  }
+  for (cudaEvent_t ev : e)
+    if (ev) cudaEventDestroy(ev);
+  return rc;
+}
+
+// The variant of epilogue ep's hop for which run() is fastest.  Variant 0 is kept unless another
+// one saves 2 % (a step with the operands out of L2 favours it slightly over the register-capped
+// ones), and the spin split (3) is taken only where it saves 3 % over the rest: back to back
+// it gains a little more than behind other kernels.
+template <typename F>
+static int tune_epilogue(int pi, int ep, F &&run) {
+  int &v = L.hop_variant[pi][ep];
+  float *t = L.hop_tune_ms[pi][ep];
+  for (v = 0; v < HOP_VARIANTS; v++) {
+    t[v] = -1.0f;
+    // 5 is slower in every measured case, 6 runs as 0 while the links are not known to come from the fundamental ones
+    if (v == 5 || (v == 6 && (L.recon12 < 3 || !L.recon_allow))) continue;
+    int rc = run();
+    if (rc == HRGPU_E_NF && v > 0) continue;  // not built for this NF
+    if (!rc) rc = time_launches(run, &t[v]);
+    if (rc) {
+      v = -1;
+      return rc;
+    }
+  }
+  v = 0;
+  auto better = [&](int c, float f) { return t[c] > 0.0f && t[c] < f * t[v]; };
+  int b = 0;
+  for (int c : {1, 2, 4, 6})
+    if (t[c] > 0.0f && t[c] < t[b]) b = c;
+  if (b && better(b, 0.98f)) v = b;
+  if (better(3, 0.97f)) v = 3;
+  return 0;
+}
+
+// the hop onto both parities of a full field: one launch of variant 1, which takes both (a
+// small lattice then fills twice the SMs), or one per parity, whichever took less time
 template <typename R>
 static int hop_full(void *out, const void *in, int ep, double cacc, const void *aux, double caux, int g5, const R *cdg,
                     const typename C2<R>::T *cod) {
-  const int v = last_hop_variant(ep, sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT);
+  const int prec = sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT, pi = tune_slot(prec);
   const size_t half = (size_t)4 * L.nf * L.ld * sizeof(typename C2<R>::T);
-  if (v == 1 && L.nf <= 6) {
+  auto one_launch = [&]() -> int {
     HopArgs<R> a;
     if (int rc = hop_args<R>(a, HRGPU_EVEN, out, in, cacc, aux, caux, g5, nullptr, cdg, cod, 0, (int)L.VH, nullptr)) return rc;
     a.both = 1;
     g_mvm += 2;
-    return launch_hop<R>(ep, a);
+    const int force = L.hop_force;
+    L.hop_force = 1;
+    const int rc = launch_hop<R>(ep, a);
+    L.hop_force = force;
+    return rc;
+  };
+  auto two_launches = [&]() -> int {
+    for (int p = 0; p < 2; p++)
+      if (int rc = hop<R>(p, (char *)out + p * half, (const char *)in + (p ^ 1) * half, ep, cacc,
+                          aux ? (const char *)aux + p * half : nullptr, caux, g5, nullptr, cdg, cod))
+        return rc;
+    return 0;
+  };
+  if (L.nf > 6) return two_launches();
+  int &both = L.hop_both[pi][ep];
+  if (both < 0 && can_tune()) {
+    const unsigned long m0 = g_mvm;
+    float t1 = 0, t2 = 0;
+    int rc = two_launches();  // tunes the hop onto one parity
+    if (!rc) rc = time_launches(two_launches, &t2);
+    if (!rc) rc = time_launches(one_launch, &t1);
+    g_mvm = m0;
+    if (rc) return rc;
+    both = t1 < t2;
   }
-  for (int p = 0; p < 2; p++)
-    if (int rc = hop<R>(p, (char *)out + p * half, (const char *)in + (p ^ 1) * half, ep, cacc,
-                        aux ? (const char *)aux + p * half : nullptr, caux, g5, nullptr, cdg, cod))
-      return rc;
-  return 0;
+  const bool b = L.hop_force >= 0 || both < 0 ? last_hop_variant(ep, prec) == 1 : both == 1;
+  return b ? one_launch() : two_launches();
 }
 
 int check_gauge(int prec) {
@@ -136,11 +221,42 @@ int Dphi_full(double m0, void *out, const void *in, int g5) {
 //            D_pp in + 1/2 D_pq tmp (clover), optionally times gamma_5.
 // Stage 1 on a range needs stage 0 done on the neighbouring range (one site
 // further in every direction).
+//
+// The variants of the two hops are chosen by the time that both take, when the second one
+// first runs on the whole parity: how well a hop follows another (what the blocks of the next
+// launch find free, what the second hop reads before the first has ended) differs between
+// variants.  The clover operator's are chosen in turn, the second with variant 0 as the first,
+// the first with that one, and the second again.
 template <typename R>
 int eo_stage(int clover, double mass, int stage, int outp, void *out, const void *in, int g5, double *red, int cb0,
              int cb1, const HopTail *tail) {
   void **tmp = sizeof(R) == 8 ? &L.tmp_o : &L.tmp_o_f;
   if (int rc = ensure_tmp(tmp, spinor_bytes(HRGPU_EVEN, sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT))) return rc;
+  const int pi = tune_slot(sizeof(R) == 8 ? HRGPU_DOUBLE : HRGPU_FLOAT);
+  const int ep0 = clover ? EP_CLOV_INV : EP_AXPY, ep1 = clover ? EP_CLOV : EP_AXPY;
+  bool &tuned = L.hop_pair_tuned[pi][clover ? 1 : 0];
+  if (!tuned && !tail && cb0 == 0 && (cb1 < 0 || cb1 == (int)L.VH) && can_tune()) {
+    if (stage == 0) {
+      if (L.hop_variant[pi][ep0] < 0) L.hop_variant[pi][ep0] = 0;  // until the second hop
+    } else {
+      const unsigned long m0 = g_mvm;
+      tuned = true;
+      auto pair = [&]() -> int {
+        if (int rc = eo_stage<R>(clover, mass, 0, outp, out, in, g5, nullptr, cb0, cb1, nullptr)) return rc;
+        return eo_stage<R>(clover, mass, 1, outp, out, in, g5, red, cb0, cb1, nullptr);
+      };
+      L.hop_variant[pi][ep0] = 0;
+      int rc = tune_epilogue(pi, ep1, pair);
+      if (!rc && clover) rc = tune_epilogue(pi, ep0, pair);
+      if (!rc && clover) rc = tune_epilogue(pi, ep1, pair);
+      if (!rc) rc = eo_stage<R>(clover, mass, 0, outp, out, in, g5, nullptr, cb0, cb1, nullptr);
+      g_mvm = m0;
+      if (rc) {
+        tuned = false;
+        return rc;
+      }
+    }
+  }
   // the second hop follows the first, which has waited for whatever made the links,
   // the clover blocks and in
   HopTail ht;
@@ -252,9 +368,18 @@ int hop_red_blocks(bool clover, int prec) {
   return v < 0 ? 0 : hop_blocks(v, L.VH, L.nf);
 }
 
+bool op_tuned(int op, int prec) {
+  if (L.hop_force >= 0) return true;
+  const bool clover = op == HRGPU_OP_G5CPHI_EOPRE_SQ || op == HRGPU_OP_G5CPHI_SQ || op == HRGPU_OP_CPHI_EOPRE ||
+                      op == HRGPU_OP_G5CPHI_EOPRE || op == HRGPU_OP_CPHI;
+  const int pi = tune_slot(prec), ep = clover ? EP_CLOV : EP_AXPY;
+  if (op_parity(op) == HRGPU_EVEN) return L.hop_pair_tuned[pi][clover];
+  return L.hop_variant[pi][ep] >= 0 && (L.nf > 6 || L.hop_both[pi][ep] >= 0);
+}
+
 bool hop_tail_settled(bool clover, int prec) {
   const int v = last_hop_variant(clover ? EP_CLOV : EP_AXPY, prec);
-  return v >= 0 && hop_tail_ok(v, L.nf, prec == HRGPU_FLOAT && L.flt_links == HRGPU_LINKS_BF16);
+  return v >= 0 && (L.hop_force >= 0 || L.hop_pair_tuned[tune_slot(prec)][clover]) && hop_tail_ok(v, L.nf, prec == HRGPU_FLOAT && L.flt_links == HRGPU_LINKS_BF16);
 }
 
 int apply_eo(bool clover, int prec, double mass, void *out, const void *in, int g5, double *red, const HopTail *tail) {

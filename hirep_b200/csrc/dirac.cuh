@@ -25,6 +25,7 @@ int apply_op(int op, int prec, double mass, void *out, const void *in);
 // tail's) partial sums of its last hop in red[0 .. hop_red_blocks(...))
 int apply_eo(bool clover, int prec, double mass, void *out, const void *in, int g5, double *red, const HopTail *tail);
 int hop_red_blocks(bool clover, int prec);  // of the variant in use; 0 while it is not tuned
+bool op_tuned(int op, int prec);  // the variants that the operator's hops use have been chosen (or forced)
 bool hop_tail_settled(bool clover, int prec);  // the variant in use is tuned and has the inverters' forms
 bool hop_small(bool clover, int prec);  // the variant in use is the one for small lattices
 void *eo_tmp(int prec);  // the even temporary of the squared operators (nullptr on failure, message set)

@@ -745,8 +745,8 @@ __device__ __forceinline__ V mul_unit(V v, int re, int im) {
 }
 
 // one thread (half h of the pair) of site cb; inactive threads compute but do
-// not write (their partner needs the shuffles)
-template <int NFT, bool REAL, typename R, int EP, typename LE = typename LinkE<REAL, R>::T>
+// not write (their partner needs the shuffles).  TAIL: as in hop_site
+template <int NFT, bool REAL, typename R, int EP, typename LE = typename LinkE<REAL, R>::T, bool TAIL = false>
 __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, const int h, const bool active) {
   typedef typename C2<R>::T V;
   typedef LE E;
@@ -809,6 +809,23 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
   double nrm = 0.0;
   V *out = (V *)a.out + cb;
   const R sg = a.g5 ? (R)-1 : (R)1;
+  // the inverters' forms: component c of the result (upper: of spins 0 and 1) and its part of the sum
+  auto put_tail = [&](int c, V v, bool upper) {
+    if (!active) return;
+    if (a.racc) {
+      V r = ((const V *)a.racc)[(long)c * ld + cb];
+      rmac(r, (R)*a.omega, v);
+      v = r;
+    }
+    out[(long)c * ld] = v;
+    if (a.red_g5) {
+      const V u = ld_c((const V *)a.aux + (long)c * ld + cb);
+      const double q = (double)u.x * v.x + (double)u.y * v.y;
+      nrm += upper ? q : -q;
+    } else {
+      nrm += (double)v.x * v.x + (double)v.y * v.y;
+    }
+  };
   if (EP == EP_AXPY) {
     // thread h writes spins h and 2+h
     const V *aux = (const V *)a.aux + cb;
@@ -820,11 +837,16 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
         rmac(o1, a.caux, ld_c(aux + (long)((2 + h) * nf + i) * ld));
       }
       o1 = cscale(sg, o1);
-      if (active) {
-        out[(long)(h * nf + i) * ld] = o0;
-        out[(long)((2 + h) * nf + i) * ld] = o1;
+      if constexpr (TAIL) {
+        put_tail(h * nf + i, o0, true);
+        put_tail((2 + h) * nf + i, o1, false);
+      } else {
+        if (active) {
+          out[(long)(h * nf + i) * ld] = o0;
+          out[(long)((2 + h) * nf + i) * ld] = o1;
+        }
+        nrm += (double)o0.x * o0.x + (double)o0.y * o0.y + (double)o1.x * o1.x + (double)o1.y * o1.y;
       }
-      nrm += (double)o0.x * o0.x + (double)o0.y * o0.y + (double)o1.x * o1.x + (double)o1.y * o1.y;
     }
   } else {
     // thread h applies clover block h: block 0 on spins (0,1), block 1 on spins (2,3)
@@ -860,24 +882,29 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
       }
       o0 = cscale(sb, o0);
       o1 = cscale(sb, o1);
-      if (active) {
-        out[(long)((2 * h) * nf + i) * ld] = o0;
-        out[(long)((2 * h + 1) * nf + i) * ld] = o1;
+      if constexpr (TAIL) {
+        put_tail((2 * h) * nf + i, o0, h == 0);
+        put_tail((2 * h + 1) * nf + i, o1, h == 0);
+      } else {
+        if (active) {
+          out[(long)((2 * h) * nf + i) * ld] = o0;
+          out[(long)((2 * h + 1) * nf + i) * ld] = o1;
+        }
+        nrm += (double)o0.x * o0.x + (double)o0.y * o0.y + (double)o1.x * o1.x + (double)o1.y * o1.y;
       }
-      nrm += (double)o0.x * o0.x + (double)o0.y * o0.y + (double)o1.x * o1.x + (double)o1.y * o1.y;
     }
   }
   return active ? nrm : 0.0;
 }
 
-template <int NFT, bool REAL, typename R, int EP, int MINB, typename LE = typename LinkE<REAL, R>::T>
+template <int NFT, bool REAL, typename R, int EP, int MINB, typename LE = typename LinkE<REAL, R>::T, bool TAIL = false>
 __global__ void __launch_bounds__(HOP_THREADS, MINB) k_hop2(HopArgs<R> a) {
   pdl_enter();
   if (a.stop && *a.stop) return;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = a.cb0 + (tid >> 1) < a.cb1;
   const int cb = active ? a.cb0 + (tid >> 1) : a.cb1 - 1;
-  double nrm = hop2_site<NFT, REAL, R, EP, LE>(a, cb, tid & 1, active);
+  double nrm = hop2_site<NFT, REAL, R, EP, LE, TAIL>(a, cb, tid & 1, active);
   if (a.red) block_partial<R>(nrm, a.red);
 }
 

@@ -57,7 +57,7 @@ inline int hop_blocks(int variant, long nsites, int nf) {
 
 // the variants whose epilogue has the inverters' forms (HopArgs::racc, red_g5)
 inline bool hop_tail_ok(int variant, int nf, bool bf16) {
-  return (!bf16 && (variant == 0 || variant == 2 || variant == 6)) || (variant == 1 && nf <= 6);
+  return (!bf16 && (variant == 0 || variant == 2 || variant == 6 || (variant == 3 && nf <= 6))) || (variant == 1 && nf <= 6);
 }
 
 __device__ __forceinline__ float hd_elem(const __nv_bfloat16 *p) { return __bfloat162float(__ldg(p)); }

@@ -111,6 +111,19 @@ int launch_dir(HopArgs<R> &a, long nsites, cudaStream_t s) {
   return 0;
 }
 
+// variant 3: two threads per site.  For NF <= 6 with the registers that it takes: capped for
+// 4 blocks per SM it was slower than that, or than variants 0 and 2, at every size from
+// 4^3 x 8 to 24^4 (2 to 6 colours, FP64 and FP32, with and without clover), while uncapped it
+// is the best one between the sizes of variant 1 and of variant 0: 20.4 us per operator against
+// 25.9 for g5Cphi of SU(4) on 10x14x12x20, 28.7 against 34.9 for the FP32 clover operator of
+// SU(4) antisymmetric.  Larger NF has it uncapped as variant 1.
+template <int N, bool RL, typename R, int EP, typename LE = typename LinkE<RL, R>::T>
+static inline void (*hop2_kernel(bool tail))(HopArgs<R>) {
+  constexpr bool T = HopDirOK<N>::v && EP != EP_CLOV_INV && std::is_same<LE, typename LinkE<RL, R>::T>::value;
+  constexpr int MINB = HopDirOK<N>::v ? 1 : 4;
+  return tail ? k_hop2<N, RL, R, EP, MINB, LE, T> : k_hop2<N, RL, R, EP, MINB, LE>;
+}
+
 // variant 6: k_hop (variant 0's register budget) building the NF = 6
 // two-index links from the fundamental ones (FP64 from L.Ug, FP32 from its
 // float copy L.Ugf) while the fundamental links are those the represented
@@ -138,8 +151,8 @@ int launch_ep_variant(HopArgs<R> &a, int variant) {
   a.nf = L.nf;
   a.recon = L.recon_allow ? L.recon12 : 0;
   // variants: 0 one thread per site, 1 one warp per direction (NF <= 6; else two threads
-  // per site, spin split), 2 as 0 and 3 the spin split with the register budget capped
-  // for 4 resident blocks per SM,
+  // per site, spin split), 2 as 0 with the register budget capped for 4 resident blocks
+  // per SM, 3 the spin split (NF > 6: capped likewise),
   // 4 one thread per site with the per-direction loads pipelined through shared memory,
   // 5 one thread per site with the time halo staged by bulk (TMA) copies,
   // 6 one thread per site building the NF = 6 two-index links from the fundamental ones
@@ -155,7 +168,7 @@ int launch_ep_variant(HopArgs<R> &a, int variant) {
       case 1:                                                                          \
         if (int rc_ = launch_dir<N, RL, R, EP>(a, nsites, s)) return rc_;              \
         break;                                                                         \
-      case 3: HR_CUDA(launch_pdl<R>(k_hop2<N, RL, R, EP, 4>, grid2, block, 0, s, a)); break; \
+      case 3: HR_CUDA(launch_pdl<R>(hop2_kernel<N, RL, R, EP>(tail), grid2, block, 0, s, a)); break; \
       case 2: HR_CUDA(launch_pdl<R>(hop_kernel<N, RL, R, EP, 4>(a.recon, tail), grid, block, 0, s, a)); break; \
       case 4:                                                                          \
         if (int rc_ = launch_async<N, RL, R, EP>(a, grid, block, s)) return rc_;       \
@@ -178,7 +191,7 @@ int launch_ep_variant(HopArgs<R> &a, int variant) {
       case 1:                                                                                   \
         if (int rc_ = launch_dir<N, RL, float, EP, typename LinkBF16<RL>::T>(a, nsites, s)) return rc_; \
         break;                                                                                  \
-      case 3: HR_CUDA(launch_pdl<float>(k_hop2<N, RL, float, EP, 4, typename LinkBF16<RL>::T>, grid2, block, 0, s, a)); break; \
+      case 3: HR_CUDA(launch_pdl<float>(hop2_kernel<N, RL, float, EP, typename LinkBF16<RL>::T>(false), grid2, block, 0, s, a)); break; \
       case 2: HR_CUDA(launch_pdl<float>(k_hop<N, RL, float, EP, 4, typename LinkBF16<RL>::T>, grid, block, 0, s, a)); break;  \
       default: return -1;                                                                       \
     }                                                                                           \
@@ -252,9 +265,10 @@ int launch_tma_checked(HopArgs<R> &a) {
 }
 
 // Autotuner: the first launch of each (precision, epilogue) on a lattice times
-// every variant on the real arguments (3 launches each, CUDA events on the
+// every variant on the real arguments (3 or 16 launches each, CUDA events on the
 // library stream) and keeps the faster one.  The output is rewritten by the
-// final launch, so tuning does not change results.  hrgpu_set_hop_variant forces
+// final launch, so tuning does not change results.  (The even-odd operators choose
+// by their two hops together, see eo_stage.)  hrgpu_set_hop_variant forces
 // a variant (tests use it to check both).
 template <typename R, int EP>
 int launch_ep(HopArgs<R> &a) {
@@ -292,6 +306,23 @@ int launch_ep(HopArgs<R> &a) {
       cudaEventDestroy(e0);
       return fail_cuda(err, "cudaEventCreate(&e1)", __FILE__, __LINE__);
     }
+    // milliseconds per launch.  A launch costs the host 2.4 to 2.8 us, as long as a hop of a
+    // small lattice takes: the launches queue up behind a delay, so that what is timed is the
+    // GPU (without it the best variant of 8 x 12 x 10 x 12 SU(2) adjoint, 3.4 us per hop, was
+    // read as 7.5 and passed over for one of 6.2).  A short hop is timed over more launches
+    // than a long one: the events resolve half a microsecond.
+    auto timed = [&](int cand, int reps, float *ms) -> int {
+      if (int rc = stream_delay(reps < 16 ? 30.0 : 80.0)) return rc;
+      if (int rc = launch_ep_variant<R, EP>(a, cand)) return rc;
+      HR_CUDA(cudaEventRecord(e0, L.stream));
+      for (int r = 0; r < reps; r++)
+        if (int rc = launch_ep_variant<R, EP>(a, cand)) return rc;
+      HR_CUDA(cudaEventRecord(e1, L.stream));
+      HR_CUDA(cudaEventSynchronize(e1));
+      HR_CUDA(cudaEventElapsedTime(ms, e0, e1));
+      *ms /= reps;
+      return 0;
+    };
     // the events are destroyed on every way out of the loop
     auto tune = [&]() -> int {
       for (int cand = 0; cand < HOP_VARIANTS; cand++) {
@@ -305,14 +336,11 @@ int launch_ep(HopArgs<R> &a) {
           continue;
         }
         if (rc0) return rc0;
-        HR_CUDA(cudaEventRecord(e0, L.stream));
-        for (int r = 0; r < 3; r++)
-          if (int rc = launch_ep_variant<R, EP>(a, cand)) return rc;
-        HR_CUDA(cudaEventRecord(e1, L.stream));
-        HR_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
-        HR_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        L.hop_tune_ms[pi][EP][cand] = ms / 3.0f;
+        if (int rc = timed(cand, 3, &ms)) return rc;
+        if (ms < 0.03f)
+          if (int rc = timed(cand, 16, &ms)) return rc;
+        L.hop_tune_ms[pi][EP][cand] = ms;
         if (ms < best) {
           best = ms;
           bestv = cand;
@@ -330,7 +358,7 @@ int launch_ep(HopArgs<R> &a) {
     // ahead with L2 flushed): another variant replaces variant 0 only when it
     // is at least 3 % faster
     const float t0 = L.hop_tune_ms[pi][EP][0];
-    if (bestv != 0 && t0 > 0.0f && best / 3.0f > 0.97f * t0) bestv = 0;
+    if (bestv != 0 && t0 > 0.0f && best > 0.97f * t0) bestv = 0;
     v = bestv;
   }
   int rc = launch_ep_variant<R, EP>(a, v);

@@ -115,6 +115,8 @@ struct Lattice {
   const int *cur_stop = nullptr;  // set by the inverters while they drive the operator
   // tuned hopping-kernel variant [FP64, FP32, FP32 with BF16 links][epilogue]
   int hop_variant[3][3] = {{-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};
+  bool hop_pair_tuned[3][2] = {};  // ... on the even-odd operator's two hops [slot][clover]
+  int hop_both[3][3] = {{-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};  // full fields: 1 both parities in a launch, 0 two launches
   int hop_force = -1;             // forced variant (-1: autotune)
   unsigned *hop_err = nullptr;    // device error word of the TMA-staged variant
   bool hop_pdl = true;            // whole-lattice hops with programmatic dependent launch
@@ -154,6 +156,8 @@ int ensure_tmp(void **p, size_t bytes);
 bool optional_room(size_t bytes);
 bool optional_allowed();
 void cg_drop_work();  // the CG's work fields
+// keeps the library's stream busy for about so many microseconds
+int stream_delay(double us);
 // a kernel's limit of dynamic shared memory raised, once per kernel and device
 int allow_smem(const void *kernel, int bytes);
 int library_device();  // the device of hrgpu_init (-1 before)

@@ -272,7 +272,7 @@ struct QMRWork {
   cudaStream_t cap = nullptr;
   // the captured iterations and what they were captured for
   cudaGraphExec_t exec = nullptr;
-  int op = -1, n = 0, v[3] = {-1, -1, -1}, force = -1, pdl = -1, recon = -1;
+  int op = -1, n = 0, v[3] = {-1, -1, -1}, force = -1, pdl = -1, recon = -1, both = -1;
   double mass = 0.0;
   const void *key[9] = {};
   void **d_ptrs = nullptr;  // out[QMAX], qa[QMAX], qb[QMAX]
@@ -334,10 +334,8 @@ static int qmr_chunk(int op, double mass, int n, void *const (&P)[3], long ne, u
   const bool clover = op == HRGPU_OP_CPHI_EOPRE || op == HRGPU_OP_CPHI;
   if (clover) QTRY(clover_prepare(mass, HRGPU_DOUBLE));
   const int *hv = L.hop_variant[0];
-  const bool settled = L.hop_force >= 0 || (clover ? (hv[EP_CLOV] >= 0 && (op == HRGPU_OP_CPHI || hv[EP_CLOV_INV] >= 0))
-                                                   : hv[EP_AXPY] >= 0);
   const unsigned long m0 = mvm_count();
-  if (!settled) {  // tunes the hopping kernels
+  if (!op_tuned(op, HRGPU_DOUBLE)) {  // tunes the hopping kernels
     const int rc = qmr_iterations(op, mass, P, ne, g);
     *mvm = mvm_count() - m0;
     mvm_restore(m0);
@@ -347,8 +345,9 @@ static int qmr_chunk(int op, double mass, int n, void *const (&P)[3], long ne, u
     QTRY(ensure_tmp(&L.tmp_o, spinor_bytes(HRGPU_EVEN, HRGPU_DOUBLE)));
   const void *key[9] = {P[0], P[1], P[2], QW.S, QW.d_ptrs, L.U, L.tmp_o, L.partials, L.cl_idg};
   const int recon = L.recon_allow ? L.recon12 : 0;
+  const int both = L.hop_both[0][clover ? EP_CLOV : EP_AXPY];
   bool same = QW.exec && QW.op == op && QW.n == n && QW.mass == mass && QW.force == L.hop_force && QW.pdl == (int)L.hop_pdl &&
-              QW.recon == recon;
+              QW.recon == recon && QW.both == both;
   for (int i = 0; i < 3 && same; i++) same = QW.v[i] == hv[i];
   for (int i = 0; i < 9 && same; i++) same = QW.key[i] == key[i];
   const unsigned long per = QMR_CHUNK * 2ul;  // two hops per application of D, even-odd or full
@@ -381,6 +380,7 @@ static int qmr_chunk(int op, double mass, int n, void *const (&P)[3], long ne, u
     QW.force = L.hop_force;
     QW.pdl = (int)L.hop_pdl;
     QW.recon = recon;
+    QW.both = both;
     for (int i = 0; i < 3; i++) QW.v[i] = hv[i];
     for (int i = 0; i < 9; i++) QW.key[i] = key[i];
   }

@@ -164,8 +164,8 @@ int hrgpu_Dphi_eopre_flt(double m0, void *out, const void *in);
 int hrgpu_g5Dphi_eopre_flt(double m0, void *out, const void *in);
 int hrgpu_g5Dphi_eopre_sq_flt(double m0, void *out, const void *in);
 /* Hopping-kernel variant: 0 = one thread per site, 1 = one warp per direction on 32
- * sites (NF <= 6; larger NF two threads per site, spin split), 2 = as 0 and 3 = spin
- * split with registers capped for 4 blocks per SM,
+ * sites (NF <= 6; larger NF two threads per site, spin split), 2 = as 0 with
+ * registers capped for 4 blocks per SM, 3 = spin split (NF > 6: capped likewise),
  * 4 = one thread per site with cp.async-pipelined loads, 5 = one thread per site
  * with the time halo staged in shared memory by bulk (TMA) copies (4 and 5: NF <= 4
  * complex, NF = 3 real; 5 also needs time slabs of a multiple of 128 sites per
@@ -173,8 +173,9 @@ int hrgpu_g5Dphi_eopre_sq_flt(double m0, void *out, const void *in);
  * antisymmetric links from the fundamental ones (link modes 3 and 4 of
  * hrgpu_link_recon; the FP32 operators from a float copy of the fundamental
  * links made with the FP32 represented ones), -1 = autotune on first use (default).  hrgpu_hop_tuning
- * reports the variant chosen for (precision, epilogue 0..2) and the per-launch
- * times it measured (ms has room for 7 values; -1 marks a variant not built for
+ * reports the variant chosen for (precision, epilogue 0..2) and the times it
+ * measured, of one launch, or once an even-odd operator has run of its two
+ * launches (ms has room for 7 values; -1 marks a variant not built for
  * this NF, lattice or link mode); precision 2 is the FP32 operator reading BF16
  * links.
  * Tuning controls of this library; they have no counterpart in the reference. */

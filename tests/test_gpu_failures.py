@@ -85,7 +85,7 @@ def test_singular_system_is_a_breakdown():
     assert status_of(e.value) == G.E_BREAKDOWN
 
 
-@pytest.mark.parametrize("variant", [-1, 0, 1, 2, 4])
+@pytest.mark.parametrize("variant", [-1, 0, 1, 2, 3, 4])
 @pytest.mark.parametrize("shifts", [[0.0], [0.0, -1.0, -3.0]])
 @pytest.mark.parametrize("flt", [False, True])
 @pytest.mark.parametrize("clover", [False, True])

@@ -1,7 +1,7 @@
-"""The hopping kernel with one warp per direction (variant 1, NF <= 6) at the sizes where
-an index could go wrong: extents of 2, parities that are no multiple of its 32 sites,
+"""The hopping kernels for small lattices, with one warp per direction (variant 1, NF <= 6) and
+with two threads per site (variant 3), at the sizes where an index could go wrong: extents of 2, parities that are no multiple of its 32 sites,
 both parities of a full field in one launch, FP32 and BF16 links; and the inverters,
-whose last hop adds to the residual (variants 0, 1, 2) or leaves it to a kernel of its
+whose last hop adds to the residual (variants 0 to 3) or leaves it to a kernel of its
 own (variant 4), against the oracle."""
 import numpy as np
 import pytest
@@ -43,12 +43,12 @@ def pin():
     lib.hrgpu_set_flt_link_storage(G.LINKS_F32)
 
 
-@pytest.mark.parametrize("represent", [True, False])
+@pytest.mark.parametrize("variant,represent", [(1, True), (1, False), (3, True)])
 @pytest.mark.parametrize("dims", DIMS)
 @pytest.mark.parametrize("ng,rep", GROUPS)
-def test_operators(ng, rep, dims, represent, pin):
+def test_operators(ng, rep, dims, variant, represent, pin):
     o, lat = setup(ng, rep, dims, True, represent)
-    pin(1)
+    pin(variant)
     e, f = F.gaussian_spinor(1, o.VH, o.nf), F.gaussian_spinor(2, o.V, o.nf)
     for name, src, par in (("Dphi_eopre", e, G.EVEN), ("g5Dphi_eopre_sq", e, G.EVEN), ("Dphi", f, G.FULL),
                            ("g5Dphi_sq", f, G.FULL), ("Cphi_eopre", e, G.EVEN), ("g5Cphi", f, G.FULL)):
@@ -65,7 +65,7 @@ def test_operators(ng, rep, dims, represent, pin):
         assert np.abs(out.download() - ref).max() < tol * np.abs(ref).max()
 
 
-@pytest.mark.parametrize("variant", [0, 1, 2, 4])
+@pytest.mark.parametrize("variant", [0, 1, 2, 3, 4])
 @pytest.mark.parametrize("clover", [False, True])
 @pytest.mark.parametrize("ng,rep", [(3, O.FUND), (2, O.ADJ)])
 def test_cg_forms(ng, rep, clover, variant, pin):
@@ -90,7 +90,7 @@ def test_cg_forms(ng, rep, clover, variant, pin):
             assert np.linalg.norm(r) < 1.1e-12 * np.linalg.norm(b), (shifts, flt)
 
 
-@pytest.mark.parametrize("variant", [0, 1, 4])
+@pytest.mark.parametrize("variant", [0, 1, 3, 4])
 @pytest.mark.parametrize("op,par", [(G.OP_DPHI_EOPRE, G.EVEN), (G.OP_CPHI_EOPRE, G.EVEN), (G.OP_DPHI, G.FULL)])
 def test_g5qmr_forms(op, par, variant, pin):
     o, lat = setup(3, O.FUND, (4, 6, 2, 4), op == G.OP_CPHI_EOPRE)
@@ -111,7 +111,7 @@ def test_g5qmr_forms(op, par, variant, pin):
             assert np.linalg.norm(b - (apply(m, xh) - s * xh)) < 1.1e-10 * np.linalg.norm(b)
 
 
-@pytest.mark.parametrize("variant", [0, 1, 4])
+@pytest.mark.parametrize("variant", [0, 1, 3, 4])
 @pytest.mark.parametrize("ng,rep", GROUPS)
 def test_g5qmr_without_a_diagonal_term(ng, rep, variant, pin):
     """m = -4: the operator has no diagonal term, but the inverter's product with its input stays."""
