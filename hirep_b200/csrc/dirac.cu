@@ -114,33 +114,58 @@ static int time_launches(F &&run, float *ms) {
   return rc;
 }
 
-// The variant of epilogue ep's hop for which run() is fastest.  Variant 0 is kept unless another
-// one saves 2 % (a step with the operands out of L2 favours it slightly over the register-capped
-// ones), and the spin split (3) is taken only where it saves 3 % over the rest: back to back
-// it gains a little more than behind other kernels.
+// run() timed with each variant for epilogue ep's hop (and too's, where not negative):
+// milliseconds, -1 where a variant is not built or not applicable
 template <typename F>
-static int tune_epilogue(int pi, int ep, F &&run) {
-  int &v = L.hop_variant[pi][ep];
+static int time_variants(int pi, int ep, int too, F &&run) {
   float *t = L.hop_tune_ms[pi][ep];
-  for (v = 0; v < HOP_VARIANTS; v++) {
+  for (int v = 0; v < HOP_VARIANTS; v++) {
     t[v] = -1.0f;
     // 5 is slower in every measured case, 6 runs as 0 while the links are not known to come from the fundamental ones
     if (v == 5 || (v == 6 && (L.recon12 < 3 || !L.recon_allow))) continue;
+    L.hop_variant[pi][ep] = v;
+    if (too >= 0) L.hop_variant[pi][too] = v;
     int rc = run();
     if (rc == HRGPU_E_NF && v > 0) continue;  // not built for this NF
     if (!rc) rc = time_launches(run, &t[v]);
-    if (rc) {
-      v = -1;
-      return rc;
-    }
+    if (rc) return rc;
   }
-  v = 0;
-  auto better = [&](int c, float f) { return t[c] > 0.0f && t[c] < f * t[v]; };
-  int b = 0;
+  return 0;
+}
+
+// The variants of an even-odd operator's two hops by the time run(), which launches both, takes:
+// how well a hop follows another (what the blocks of the next launch find free, what the
+// second hop reads before the first has ended) differs between variants.  The same variant
+// for both hops first: 0 unless another one saves 2 % (a step with the operands out of L2
+// favours it slightly over the register-capped ones), and the spin split (3) only where it saves
+// 3 % over the rest.  A second one beside it only where that saves 2 % (sextet clover at
+// 48x24^3: 763 us with 6 and 1, 860 and 868 with one of them), or 8 % of less than 100 us: the
+// gaps between short launches are others behind other kernels than back to back (g5QMR
+// with clover, SU(3) on 12x6x14x10: 1 and 3 read 6 % faster than 1 and 1, and the solve took
+// 2 % more).
+template <typename F>
+static int tune_pair(int pi, int ep0, int ep1, F &&run) {
+  int &v0 = L.hop_variant[pi][ep0], &v1 = L.hop_variant[pi][ep1];
+  const float *t0 = L.hop_tune_ms[pi][ep0], *t1 = L.hop_tune_ms[pi][ep1];
+  auto best_of = [](const float *t, int from, float f) {
+    int b = from;
+    for (int c : {0, 1, 2, 4, 6, 3})
+      if (t[c] > 0.0f && t[c] < t[b]) b = c;
+    return t[b] < f * t[from] ? b : from;
+  };
+  if (int rc = time_variants(pi, ep1, ep0, run)) return rc;
+  int u = 0;
   for (int c : {1, 2, 4, 6})
-    if (t[c] > 0.0f && t[c] < t[b]) b = c;
-  if (b && better(b, 0.98f)) v = b;
-  if (better(3, 0.97f)) v = 3;
+    if (t1[c] > 0.0f && t1[c] < t1[u]) u = c;
+  if (t1[u] > 0.98f * t1[0]) u = 0;
+  if (t1[3] > 0.0f && t1[3] < 0.97f * t1[u]) u = 3;
+  v0 = v1 = u;
+  if (ep0 == ep1) return 0;
+  if (int rc = time_variants(pi, ep1, -1, run)) return rc;
+  const float f = t1[u] > 0.1f ? 0.98f : 0.92f;
+  v1 = best_of(t1, u, f);
+  if (int rc = time_variants(pi, ep0, -1, run)) return rc;
+  v0 = best_of(t0, u, v1 == u ? f : 0.98f);
   return 0;
 }
 
@@ -222,11 +247,8 @@ int Dphi_full(double m0, void *out, const void *in, int g5) {
 // Stage 1 on a range needs stage 0 done on the neighbouring range (one site
 // further in every direction).
 //
-// The variants of the two hops are chosen by the time that both take, when the second one
-// first runs on the whole parity: how well a hop follows another (what the blocks of the next
-// launch find free, what the second hop reads before the first has ended) differs between
-// variants.  The clover operator's are chosen in turn, the second with variant 0 as the first,
-// the first with that one, and the second again.
+// The variants of the two hops are chosen (tune_pair) when the second one first runs on the
+// whole parity.
 template <typename R>
 int eo_stage(int clover, double mass, int stage, int outp, void *out, const void *in, int g5, double *red, int cb0,
              int cb1, const HopTail *tail) {
@@ -245,14 +267,12 @@ int eo_stage(int clover, double mass, int stage, int outp, void *out, const void
         if (int rc = eo_stage<R>(clover, mass, 0, outp, out, in, g5, nullptr, cb0, cb1, nullptr)) return rc;
         return eo_stage<R>(clover, mass, 1, outp, out, in, g5, red, cb0, cb1, nullptr);
       };
-      L.hop_variant[pi][ep0] = 0;
-      int rc = tune_epilogue(pi, ep1, pair);
-      if (!rc && clover) rc = tune_epilogue(pi, ep0, pair);
-      if (!rc && clover) rc = tune_epilogue(pi, ep1, pair);
+      int rc = tune_pair(pi, ep0, ep1, pair);
       if (!rc) rc = eo_stage<R>(clover, mass, 0, outp, out, in, g5, nullptr, cb0, cb1, nullptr);
       g_mvm = m0;
       if (rc) {
         tuned = false;
+        L.hop_variant[pi][ep0] = L.hop_variant[pi][ep1] = -1;
         return rc;
       }
     }
