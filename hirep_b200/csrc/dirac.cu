@@ -138,7 +138,8 @@ static int time_variants(int pi, int ep, int too, F &&run) {
 // second hop reads before the first has ended) differs between variants.  The same variant
 // for both hops first: 0 unless another one saves 2 % (a step with the operands out of L2
 // favours it slightly over the register-capped ones), and the spin split (3) only where it saves
-// 3 % over the rest.  A second one beside it only where that saves 2 % (sextet clover at
+// 6 % over the rest (inside a solve it gains less: g5QMR with clover, SU(4) on 6x10x12x16,
+// took 2 % more with it than with 1 where the pair read less).  A second one beside it only where that saves 2 % (sextet clover at
 // 48x24^3: 763 us with 6 and 1, 860 and 868 with one of them), or 8 % of less than 100 us: the
 // gaps between short launches are others behind other kernels than back to back (g5QMR
 // with clover, SU(3) on 12x6x14x10: 1 and 3 read 6 % faster than 1 and 1, and the solve took
@@ -158,7 +159,7 @@ static int tune_pair(int pi, int ep0, int ep1, F &&run) {
   for (int c : {1, 2, 4, 6})
     if (t1[c] > 0.0f && t1[c] < t1[u]) u = c;
   if (t1[u] > 0.98f * t1[0]) u = 0;
-  if (t1[3] > 0.0f && t1[3] < 0.97f * t1[u]) u = 3;
+  if (t1[3] > 0.0f && t1[3] < 0.94f * t1[u]) u = 3;
   v0 = v1 = u;
   if (ep0 == ep1) return 0;
   if (int rc = time_variants(pi, ep1, -1, run)) return rc;

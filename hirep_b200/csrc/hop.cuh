@@ -809,18 +809,27 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
   double nrm = 0.0;
   V *out = (V *)a.out + cb;
   const R sg = a.g5 ? (R)-1 : (R)1;
-  // the inverters' forms: component c of the result (upper: of spins 0 and 1) and its part of the sum
-  auto put_tail = [&](int c, V v, bool upper) {
-    if (!active) return;
-    if (a.racc) {
-      V r = ((const V *)a.racc)[(long)c * ld + cb];
-      rmac(r, (R)*a.omega, v);
-      v = r;
+  // the inverters' forms: the thread's components c0 + i and c1 + i of the residual or of aux,
+  // loaded before the first store (out may be the residual, so no load passes a store)
+  V w0[TAIL ? NA : 1], w1[TAIL ? NA : 1];
+  auto load_tail = [&](int c0, int c1) {
+    const V *w = (const V *)(a.racc ? a.racc : a.aux) + cb;
+#pragma unroll
+    for (int i = 0; i < (TAIL ? NA : 0); i++) {
+      w0[i] = active ? w[(long)(c0 + i) * ld] : cmk<V>(0.0, 0.0);
+      w1[i] = active ? w[(long)(c1 + i) * ld] : cmk<V>(0.0, 0.0);
     }
-    out[(long)c * ld] = v;
+  };
+  // component c of the result (upper: of spins 0 and 1), w its element
+  const R om = TAIL && a.racc ? (R)*a.omega : (R)0;
+  auto put_tail = [&](int c, V v, V w, bool upper) {
+    if (a.racc) {
+      rmac(w, om, v);
+      v = w;
+    }
+    if (active) out[(long)c * ld] = v;
     if (a.red_g5) {
-      const V u = ld_c((const V *)a.aux + (long)c * ld + cb);
-      const double q = (double)u.x * v.x + (double)u.y * v.y;
+      const double q = (double)w.x * v.x + (double)w.y * v.y;
       nrm += upper ? q : -q;
     } else {
       nrm += (double)v.x * v.x + (double)v.y * v.y;
@@ -829,6 +838,7 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
   if (EP == EP_AXPY) {
     // thread h writes spins h and 2+h
     const V *aux = (const V *)a.aux + cb;
+    if constexpr (TAIL) load_tail(h * nf, (2 + h) * nf);
 #pragma unroll
     for (int i = 0; i < NA; i++) {
       V o0 = cscale(ca, rm[i]), o1 = cscale(ca, h ? p3[i] : p2[i]);
@@ -838,8 +848,8 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
       }
       o1 = cscale(sg, o1);
       if constexpr (TAIL) {
-        put_tail(h * nf + i, o0, true);
-        put_tail((2 + h) * nf + i, o1, false);
+        put_tail(h * nf + i, o0, w0[i], true);
+        put_tail((2 + h) * nf + i, o1, w1[i], false);
       } else {
         if (active) {
           out[(long)(h * nf + i) * ld] = o0;
@@ -873,6 +883,7 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
     }
     herm_apply<NA, 1>(yout, xin, a.cdg + (long)h * n2 * lp, a.cod + (long)h * no * lp, lp, site, nf);
     const R sb = h ? sg : (R)1;
+    if constexpr (TAIL) load_tail((2 * h) * nf, (2 * h + 1) * nf);
 #pragma unroll
     for (int i = 0; i < NA; i++) {
       V o0 = yout[i], o1 = yout[nf + i];
@@ -883,8 +894,8 @@ __device__ __forceinline__ double hop2_site(const HopArgs<R> &a, const int cb, c
       o0 = cscale(sb, o0);
       o1 = cscale(sb, o1);
       if constexpr (TAIL) {
-        put_tail((2 * h) * nf + i, o0, h == 0);
-        put_tail((2 * h + 1) * nf + i, o1, h == 0);
+        put_tail((2 * h) * nf + i, o0, w0[i], h == 0);
+        put_tail((2 * h + 1) * nf + i, o1, w1[i], h == 0);
       } else {
         if (active) {
           out[(long)((2 * h) * nf + i) * ld] = o0;
