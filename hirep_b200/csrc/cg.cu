@@ -194,8 +194,9 @@ struct CGRing {
 // The iterations kept in S (pend of them, their residuals in ring) applied to every shifted
 // system: x_i += cx p_i, p_i = cp p_i + pz r, one after the other in registers, so the
 // results are bit for bit those of an update in each iteration.  Such an update is bound by HBM:
-// 4n + 3 vectors per iteration (76 us, 6.6 TB/s, for 10 shifts on 16^4 with NF=6 in FP64);
-// this is 4n + CG_CHUNK per CG_CHUNK iterations, with k alone in between.
+// 4n + 1 vectors in each; this is 4n + CG_CHUNK per CG_CHUNK iterations.  The solve with 10
+// shifts on 16^4 with NF = 6 in FP64 takes 17.5 ms, and 23.5 ms with an update in each iteration
+// (516 MB, part of it still in L2).
 template <typename W, typename R>
 __global__ void __launch_bounds__(RED_THREADS) k_cg_shifts(const CGState *S, W *const *x, W *const *p, CGRing<W> ring, long n) {
   const int pend = S->pend;
@@ -325,8 +326,8 @@ static bool cg_more_residuals(CGWork &w, int nvec) {
 }
 
 // The chunk of iterations as a CUDA graph, captured once per (operator, mass,
-// work buffers, kernel variants, link storage) and replayed: eight launches per
-// iteration, most of them small, cost more in launch gaps than in work.  The
+// work buffers, kernel variants, link storage) and replayed: seven launches per
+// iteration (one more every CG_CHUNK with shifted systems), most of them small, cost more in launch gaps than in work.  The
 // graph reads the links and clover blocks at replay; the clover blocks (for
 // this mass) and the BF16 link copy are brought up to date before each replay.
 // (Folding the partials in the last block of the kernel that wrote them, with

@@ -384,7 +384,11 @@ __global__ void k_clover_pack_inv(const double2 *cl, double sigma, double *dg, d
 // one row of 2NF complex in each lane's registers, and inverts it in place by
 // Gauss-Jordan steps without pivoting (the pivots are the D of the LDL
 // factorisation, and their product the determinant): step k's pivot row goes
-// through shared memory and every lane takes its multiple off its own row.  A
+// through shared memory and every lane takes its multiple off its own row.  The
+// eigenvalues of A are below 1.4 csw in size on Haar-random links, so D is positive for the
+// masses in use, and the error is then that of the LDL solves or less (random matrices of
+// condition 10 to 1e9); for an indefinite D, where neither is stable, its median is
+// 1.7 times theirs.  A
 // thread block is 8 sites, both chiral blocks of each: the clover term comes in and
 // the packed blocks go out through shared memory as runs of 8 sites (128 bytes).
 // Bound by the steps' shared-memory reads (12 of 16 bytes per lane and step at NF = 6)

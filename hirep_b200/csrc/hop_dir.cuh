@@ -14,11 +14,12 @@
 // (8^4 has 16 blocks of 128 sites for 148 SMs), and the NF = 6 clover hop, whose
 // 144 clover numbers per site it loads by eight warps.  A large NF = 3 lattice is bound
 // by HBM and L2, where 128 consecutive sites per block share their y neighbours in L1
-// and 32 do not.  Per hop, FP64, against the best of the other variants:
-//   8^4 SU(3)                          4.4 us, 6.7 (spin split 5.1 before)
-//   14x6x10x12 SU(4) antisymmetric    11.3 us, 17.8
-//   48x24^3 SU(3) sextet, clover       436 us, 482
-//   32x16^3 SU(3), clover               38 us, 21 (the autotuner keeps the others)
+// and 32 do not.  Per operator, FP64, in a CUDA graph of many, against the best of the others:
+//   8^4 SU(3) Dphi_eopre                        5.2 us, 6.7 (two threads per site)
+//   14x6x10x12 SU(4) antisymmetric g5Dphi_sq   28.4 us, 38.2
+//   48x24^3 SU(3) sextet Cphi_eopre             868 us, 839 (links built from the fundamental
+//                                                ones, as here); 769 with that hop first
+//   32x16^3 SU(3) Cphi_eopre                   75.7 us, 39 (the autotuner keeps the others)
 // What bounds it: the latency of one load from L2, two barriers and the launch.  Of two
 // hops of an operator the second reads its links, clover blocks and diagonal-term field
 // while the first still runs (programmatic dependent launch), and waits for it only

@@ -13,7 +13,8 @@ namespace hrgpu {
 // (the kernels wait on their predecessor with griddepcontrol.wait before
 // reading memory), so its blocks fill the SMs the previous hop's last wave
 // leaves idle: Cphi_eopre 62.5 -> 60.4 us at 16^3x32 (alternating A/B in one
-// process), the FP64 CG unchanged.  Without it: FP32 hops (inside the mixed
+// process), the FP64 CG unchanged.  small: variant 1, whose launches overlap in FP32
+// as well.  Without it: the other FP32 hops (inside the mixed
 // solve's graphs it cost 3 %: 18.7 -> 19.3 ms) and launches over a few time
 // slabs (the host-field pipeline, where the early, waiting blocks held SMs
 // that the copy-stream kernels beside them needed: 0.47 -> 0.69 ms).

@@ -181,7 +181,7 @@ int hrgpu_g5Dphi_eopre_sq_flt(double m0, void *out, const void *in);
  * Tuning controls of this library; they have no counterpart in the reference. */
 int hrgpu_set_hop_variant(int variant);
 int hrgpu_hop_tuning(int prec, int epilogue, int *chosen, float *ms);
-/* whole-lattice FP64 hopping kernels launched with programmatic dependent
+/* whole-lattice FP64 hopping kernels (and FP32 ones of variant 1) launched with programmatic dependent
  * launch (default 1: the next hop's blocks start in the SMs the previous hop's
  * last wave leaves idle); 0 launches them plainly */
 int hrgpu_set_hop_pdl(int on);
