@@ -3,8 +3,11 @@ with two threads per site (variant 3), at the sizes where an index could go wron
 both parities of a full field in one launch, FP32 and BF16 links; and the inverters,
 whose last hop adds to the residual (variants 0 to 3) or leaves it to a kernel of its
 own (variant 4), against the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
 import oracle as O
 from hirep_b200 import fields as F
@@ -156,3 +159,56 @@ def test_reads_the_stored_links(ng, rep, pin):
             assert np.array_equal(out.download(), full.download()), name
     finally:
         lat.L.hrgpu_set_link_recon(1)
+
+
+@pytest.mark.parametrize("ng,rep", [(3, O.FUND), (2, O.ADJ), (4, O.ASYM), (4, O.SYM)])
+def test_choice_of_variants(ng, rep, pin):
+    """The first calls on a lattice choose the variants (a call that is captured cannot, and runs
+    without): captured first, choosing and chosen, each call gives the operator's result and
+    counts its hops as any other does."""
+    o, lat = setup(ng, rep, (4, 6, 2, 10), True)
+    e, f = F.gaussian_spinor(1, o.VH, o.nf), F.gaussian_spinor(2, o.V, o.nf)
+    calls = []
+    for name, src, par, prec, mvm in (("Dphi_eopre", e, G.EVEN, G.DOUBLE, 1), ("g5Cphi_eopre_sq", e, G.EVEN, G.DOUBLE, 2),
+                                      ("g5Dphi_sq", f, G.FULL, G.DOUBLE, 2), ("Cphi", f, G.FULL, G.DOUBLE, 1),
+                                      ("Dphi_eopre_flt", e, G.EVEN, G.FLOAT, 1), ("g5Cphi_eopre_flt", e, G.EVEN, G.FLOAT, 1),
+                                      ("g5Dphi_flt", f, G.FULL, G.FLOAT, 1)):
+        host = src if prec == G.DOUBLE else src.astype(np.complex64)
+        ref = getattr(o, name[:-4] if prec == G.FLOAT else name)(M, src)
+        calls.append((name, lat.field(par, prec, host=host), lat.field(par, prec), ref, mvm))
+    pin(0)
+    for name, fin, out, _, _ in calls:  # the temporaries
+        getattr(lat, name)(M, out, fin)
+    pin(-1)
+    lat.sync()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+
+    def check():
+        for name, fin, out, ref, _ in calls:
+            # a few roundings of the largest entry per product, as in test_operators
+            tol = 4e-15 * o.nf if out.prec == G.DOUBLE else 4e-6
+            assert np.abs(out.download() - ref).max() < tol * np.abs(ref).max(), name
+            out.buf.zero_()
+
+    lat.L.hrgpu_set_stream(ctypes.c_void_p(stream.cuda_stream))
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            for name, fin, out, _, _ in calls:
+                getattr(lat, name)(M, out, fin)
+    finally:
+        lat.L.hrgpu_set_stream(ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    for name, fin, out, _, _ in calls:
+        out.buf.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    check()
+    for _ in range(2):  # choosing, chosen
+        for name, fin, out, _, mvm in calls:
+            lat.getMVM()
+            getattr(lat, name)(M, out, fin)
+            assert lat.getMVM() == mvm, name
+        lat.sync()
+        check()
+    graph.replay()
+    torch.cuda.synchronize()
+    check()
